@@ -12,6 +12,7 @@
 #include "exact.cuh"
 #include "batched.cuh"
 #include "mlp.cuh"
+#include "filter.cuh"
 #include "fuzzy.cuh"
 #include "kernels.cuh"
 #include "primitives.cuh"
@@ -769,6 +770,43 @@ int check_neighbors(pq_ctx* c, uint64_t n, uint64_t d, uint64_t nn, int32_t metr
     return PQ_OK;
 }
 
+// The tensor-core filter in front of the exact search, where it applies; false
+// when it does not (or its workspace does not fit: the full search needs none).
+bool prepare_exact_filter(pq_ctx* c, const float* X, uint64_t n, uint64_t d, uint64_t kws,
+                          int32_t metric, const float* norms, uint32_t* indices, float* dists,
+                          pq::ExactFilter* out) {
+    if (kws < 2 || !pq::filter_takes(n, d, kws)) return false;
+    try {
+        pq::FilterCall f{};
+        f.X = X;
+        f.rows = n;
+        f.d = int(d);
+        f.mode = metric == PQ_METRIC_COSINE ? pq::FILTER_COSINE : pq::FILTER_EUCLIDEAN;
+        f.norms = metric == PQ_METRIC_COSINE ? norms : nullptr;
+        pq::FilterSample s{};
+        s.n = uint32_t(n);
+        s.k = uint32_t(kws);
+        f.samples.push_back(s);
+        f.out_idx = indices;
+        f.out_dist = dists;
+        out->redo = f.redo_a = c->get<uint32_t>("ex_redo", n);
+        out->redo_n = f.redo_count = c->get<uint32_t>("ex_redo_n", 1);
+        pq::FilterPlan plan = pq::filter_prepare(c, std::move(f));
+        out->run = plan.run;
+        out->Xt = plan.Xt;
+        // distances of an eighth of the queries, in at most 1 GB (a whole number
+        // of fours)
+        const uint64_t ld = (n + 31) / 32 * 32;
+        out->redo_ld = uint32_t(ld);
+        out->redo_cap = uint32_t(std::max<uint64_t>(
+            64, std::min<uint64_t>((n + 7) / 8, (uint64_t(1) << 30) / (ld * 4)) / 4 * 4));
+        out->redo_dist = c->get<float>("ex_redo_d", out->redo_cap * ld);
+        return true;
+    } catch (const std::string&) {
+        return false;
+    }
+}
+
 // Runs f, mapping its exceptions to status codes.  On an error both of the
 // context's streams are drained before returning, so no copy into the
 // caller's buffers is still in flight when the caller sees the status.
@@ -1001,8 +1039,10 @@ int pq_neighbors_into(pq_ctx* c, const float* data, uint64_t n, uint64_t d,
         float* ddx = c->get<float>("out_dists", std::max<uint64_t>(nnz, 1));
         ck(cudaMemcpyAsync(X, data, n * d * 4, cudaMemcpyHostToDevice, st), "h2d");
         ck(pq::exact_knn_prepare(), "exact kNN set-up");
+        pq::ExactFilter flt;
+        const bool fl = prepare_exact_filter(c, X, n, d, kws, metric, norms, dix, ddx, &flt);
         ck(pq::launch_exact_knn(X, n, int(d), int(kws), metric == PQ_METRIC_COSINE, norms, dip, dix,
-                            ddx, st),
+                            ddx, st, fl ? &flt : nullptr),
            "exact kNN");
         ck(cudaMemcpyAsync(indptr, dip, (n + 1) * 4, cudaMemcpyDeviceToHost, st), "d2h");
         if (nnz) {
@@ -1032,8 +1072,11 @@ int pq_neighbors_into_device(pq_ctx* c, const float* d_data, uint64_t n, uint64_
         ck(cudaEventRecord(ev, user), "event");
         ck(cudaStreamWaitEvent(c->stream, ev, 0), "event");
         ck(pq::exact_knn_prepare(), "exact kNN set-up");
+        pq::ExactFilter flt;
+        const bool fl =
+            prepare_exact_filter(c, d_data, n, d, kws, metric, norms, d_indices, d_dists, &flt);
         ck(pq::launch_exact_knn(d_data, n, int(d), int(kws), metric == PQ_METRIC_COSINE, norms,
-                            d_indptr, d_indices, d_dists, c->stream),
+                            d_indptr, d_indices, d_dists, c->stream, fl ? &flt : nullptr),
            "exact kNN");
         ck(cudaEventRecord(ev, c->stream), "event");
         ck(cudaStreamWaitEvent(user, ev, 0), "event");
@@ -1125,8 +1168,22 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
         const uint64_t key = (d <= 32 ? 32ull : 64ull) << 32 | uint64_t(kp);
         auto it = c->batch_shape.find(key);
         int shape = -1;
+        // samples the tensor-core filter takes; the full search gets the rest,
+        // and the query blocks the filter leaves (usually none)
+        std::vector<uint8_t> taken(n_samples, 0);
+        uint64_t n_taken = 0;
+        for (uint32_t s = 0; s < n_samples; ++s) {
+            taken[s] = offsets[n_samples] < (uint64_t(1) << 30) &&
+                       pq::filter_takes(offsets[s + 1] - offsets[s], d, ks[s]);
+            n_taken += taken[s];
+        }
         if (it != c->batch_shape.end() && !(flags & PQ_BATCH_AUTOTUNE)) {
             shape = it->second;
+        } else if (n_taken == n_samples && !(flags & PQ_BATCH_AUTOTUNE)) {
+            // only left-over blocks would use the shape: not worth timing
+            for (int sh = pq::batched_shapes() - 1; sh >= 0 && shape < 0; --sh)
+                if (pq::batched_shape_fits(sh, int(d), kp)) shape = sh;
+            if (shape < 0) throw DeviceError{"no tile shape fits this k and n_dim"};
         } else {
             float best = 0.f;
             cudaEvent_t e0, e1;
@@ -1159,8 +1216,79 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
             if (shape < 0) throw DeviceError{"no tile shape fits this k and n_dim"};
             c->batch_shape[key] = shape;
         }
-        items_for(shape, is, iq);
-        upload_items(uint32_t(is.size()));
+        std::function<cudaError_t(cudaStream_t)> filter;
+        if (n_taken > 0) {
+            try {
+                items_for(shape, is, iq);
+                const size_t all_items = is.size();
+                uint32_t* redo_s = c->get<uint32_t>("bt_redo_s", all_items);
+                uint32_t* redo_q = c->get<uint32_t>("bt_redo_q", all_items);
+                uint32_t* redo_n = c->get<uint32_t>("bt_redo_n", 2);  // blocks, single queries
+                // (a group whose rows the filter cannot bound has more queries)
+                const uint32_t few = 512;
+                uint2* redo_1 = c->get<uint2>("bt_redo_1", few);
+                pq::FilterCall f{};
+                f.X = d_data;
+                f.rows = offsets[n_samples];
+                f.d = int(d);
+                f.mode = pq::FILTER_BATCHED;
+                for (uint32_t s = 0; s < n_samples; ++s) {
+                    if (!taken[s]) continue;
+                    pq::FilterSample g{};
+                    g.base = offsets[s];
+                    g.out = s_out[s];
+                    g.n = uint32_t(offsets[s + 1] - offsets[s]);
+                    g.k = ks[s];
+                    f.samples.push_back(g);
+                    f.ids.push_back(s);
+                }
+                f.out_idx = d_indices;
+                f.out_dist = d_dists;
+                f.redo_block = uint32_t(pq::batched_queries_per_item(shape));
+                f.redo_a = redo_s;
+                f.redo_b = redo_q;
+                f.redo_count = redo_n;
+                f.redo_queries = redo_1;
+                f.redo_queries_n = redo_n + 1;
+                f.redo_short = few;
+                filter = pq::filter_prepare(c, std::move(f)).run;
+                // the full search's items of the samples it takes whole, at the
+                // head of the list; the filter appends to them
+                size_t o = 0;
+                for (size_t i = 0; i < is.size(); ++i)
+                    if (!taken[is[i]]) {
+                        is[o] = is[i];
+                        iq[o++] = iq[i];
+                    }
+                is.resize(o);
+                iq.resize(o);
+                uint32_t* first = c->get<uint32_t>("bt_first_n", 2);
+                const uint32_t o32[2] = {uint32_t(o), 0u};
+                ck(cudaMemcpyAsync(first, o32, 8, cudaMemcpyHostToDevice, st), "h2d");
+                ck(cudaMemcpyAsync(redo_s, is.data(), o * 4, cudaMemcpyHostToDevice, st), "h2d");
+                ck(cudaMemcpyAsync(redo_q, iq.data(), o * 4, cudaMemcpyHostToDevice, st), "h2d");
+                b.item_s = redo_s;
+                b.item_q = redo_q;
+                b.n_items = uint32_t(all_items);
+                b.items_dev = redo_n;
+                b.first_dev = first;
+                b.single = redo_1;
+                b.single_n = redo_n + 1;
+                b.single_max = few;
+                auto run = filter;
+                filter = [=](cudaStream_t q) {
+                    cudaError_t e = cudaMemcpyAsync(redo_n, first, 8, cudaMemcpyDeviceToDevice, q);
+                    return e == cudaSuccess ? run(q) : e;
+                };
+            } catch (const std::string&) {  // no room for the filter's workspace
+                filter = nullptr;
+                b.items_dev = nullptr;
+            }
+        }
+        if (!filter) {
+            items_for(shape, is, iq);
+            upload_items(uint32_t(is.size()));
+        }
         if (flags & PQ_BATCH_GRAPH) {
             cudaStream_t cs;
             ck(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream");
@@ -1169,9 +1297,12 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
             ck(cudaStreamSynchronize(st), "items");
             ck(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
             cudaMemsetAsync(counter, 0, 4, cs);
-            pq::launch_batched_knn(b, shape, cs);
-            const cudaError_t ce = cudaStreamEndCapture(cs, &g);
+            cudaError_t le = filter ? filter(cs) : cudaSuccess;
+            if (le == cudaSuccess) le = pq::launch_batched_knn(b, shape, cs);
+            cudaError_t ce = cudaStreamEndCapture(cs, &g);
+            if (ce == cudaSuccess) ce = le;
             if (ce != cudaSuccess) {
+                if (g) cudaGraphDestroy(g);
                 cudaStreamDestroy(cs);
                 ck(ce, "capture");
             }
@@ -1183,6 +1314,7 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
             cudaStreamDestroy(cs);
         } else {
             ck(cudaMemsetAsync(counter, 0, 4, st), "counter");
+            if (filter) ck(filter(st), "batched kNN filter");
             ck(pq::launch_batched_knn(b, shape, st), "batched kNN");
         }
         ck(cudaEventRecord(ev, st), "event");

@@ -22,6 +22,10 @@
 // by a warp bitonic network at the end.  Either way the result is the exact k
 // smallest keys.  The tile shape (QW, NW) is chosen by an autotuner that
 // times each shape on the largest work items of the call.
+//
+// This full search takes the samples the tensor-core filter (filter.cu) does
+// not: d > 62 or fewer than 16 points per neighbour; and the query blocks that
+// the filter leaves, whose number only the device knows (items_dev).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,6 +51,13 @@ struct BatchArgs {
     const uint32_t* item_s;  // work item: sample
     const uint32_t* item_q;  // work item: first local query
     uint32_t n_items;
+    // optional: the number of items, on the device; items past the first
+    // *first_dev only when *single_n queries are too many for k_batched_redo
+    const uint32_t* items_dev;
+    const uint32_t* first_dev;
+    const uint2* single;
+    const uint32_t* single_n;
+    uint32_t single_max;
     uint32_t* counter;       // next work item (starts at zero)
     int kp;                  // heap capacity per query: power of two >= max k
     uint32_t* out_idx;
@@ -141,12 +152,14 @@ __global__ void __launch_bounds__(NW * 32) k_batched_knn(BatchArgs a) {
     __shared__ uint32_t s_item;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kp = a.kp;
+    const uint32_t n_items = !a.items_dev ? a.n_items
+                             : *a.single_n < a.single_max ? *a.first_dev : *a.items_dev;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1u);
         __syncthreads();
         const uint32_t item = s_item;
         __syncthreads();
-        if (item >= a.n_items) break;
+        if (item >= n_items) break;
         const uint32_t s = a.item_s[item], q0 = a.item_q[item];
         const uint64_t base = a.s_off[s];
         const uint32_t ns = uint32_t(a.s_off[s + 1] - base);
@@ -304,6 +317,90 @@ __global__ void __launch_bounds__(NW * 32) k_batched_knn(BatchArgs a) {
     }
 }
 
+// A few single queries, one CTA each (lists of the filter that overflowed): 16
+// warps evaluate 512 distances at a time and a 17th keeps the k smallest keys
+// of the previous tile.  A block of the full search would take tens of
+// milliseconds alone on a large sample, whatever the number of its queries.
+constexpr int RW = 512;
+
+__global__ void __launch_bounds__(RW + 32) k_batched_redo(BatchArgs a) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint64_t* h = reinterpret_cast<uint64_t*>(smem);  // kp keys
+    __shared__ float sq[64];
+    __shared__ float sd[2][RW];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t nq = *a.single_n;
+    if (nq >= a.single_max) return;
+    for (uint32_t i = blockIdx.x; i < nq; i += gridDim.x) {
+        const uint32_t s = a.single[i].x, q = a.single[i].y;
+        const uint64_t base = a.s_off[s];
+        const uint32_t n = uint32_t(a.s_off[s + 1] - base), tiles = (n + RW - 1) / RW;
+        const int k = int(a.s_k[s]);
+        __syncthreads();  // the previous query is finished
+        if (tid < a.d) sq[tid] = a.X[(base + q) * uint64_t(a.d) + tid];
+        __syncthreads();
+        int len = 0;
+        for (uint32_t t = 0; t <= tiles; ++t) {
+            if (tid < RW) {
+                const uint32_t j = t * RW + tid;
+                if (t < tiles && j < n) {
+                    const float* x = a.X + (base + j) * uint64_t(a.d);
+                    float acc = 0.0f;
+#pragma unroll 8
+                    for (int c = 0; c < a.d; ++c) {
+                        const float df = sq[c] - x[c];
+                        acc = fmaf(df, df, acc);
+                    }
+                    sd[t & 1][tid] = acc;
+                }
+            } else if (t > 0) {
+                for (uint32_t u = 0; u < uint32_t(RW); u += 32) {
+                    const uint32_t j = (t - 1) * RW + u + lane;
+                    const uint64_t key = dkey(sd[(t - 1) & 1][u + lane], j);
+                    uint32_t pending = __ballot_sync(FULL, j < n && j != q);
+                    while (pending && len < k) {  // the first k are pushed in order
+                        const int l = __ffs(pending) - 1;
+                        pending &= pending - 1;
+                        const uint64_t x = __shfl_sync(FULL, key, l);
+                        if (lane == 0) {
+                            h[len] = x;
+                            heap_up(h, len);
+                        }
+                        ++len;
+                        __syncwarp();
+                    }
+                    while (pending) {
+                        const uint64_t root = h[0];
+                        const uint32_t m =
+                            __ballot_sync(FULL, ((pending >> lane) & 1u) && key < root);
+                        if (!m) break;
+                        const int l = __ffs(m) - 1;
+                        pending &= (l == 31) ? 0u : ~((2u << l) - 1u);
+                        const uint64_t x = __shfl_sync(FULL, key, l);
+                        if (lane == 0) {
+                            h[0] = x;
+                            heap_down(h, len);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (tid >= RW) {
+            sort_keys(h, len, a.kp, lane);
+            const uint64_t o = a.s_out[s] + uint64_t(q) * uint64_t(k);
+            for (int t = lane; t < k; t += 32) {
+                const uint64_t v = h[t];
+                const bool ok = t < len;
+                a.out_idx[o + t] = ok ? uint32_t(v) : 0xFFFFFFFFu;
+                a.out_dist[o + t] = ok ? __fsqrt_rn(__uint_as_float(uint32_t(v >> 32)))
+                                       : __int_as_float(0x7f800000);
+            }
+        }
+    }
+}
+
 template <int DP, int QW, int NW, int KPL>
 size_t smem_bytes(int kp) {
     return size_t(NW) * DP * QW * 4 + size_t((DP * ETP + 1) & ~1) * 4 +
@@ -384,10 +481,20 @@ cudaError_t launch_batched_knn(const BatchLaunch& b, int shape, cudaStream_t st)
     a.item_s = b.item_s;
     a.item_q = b.item_q;
     a.n_items = b.n_items;
+    a.items_dev = b.items_dev;
+    a.first_dev = b.first_dev;
+    a.single = b.single;
+    a.single_n = b.single_n;
+    a.single_max = b.single_max;
     a.counter = b.counter;
     a.kp = b.kp;
     a.out_idx = b.out_idx;
     a.out_dist = b.out_dist;
+    if (b.items_dev) {
+        k_batched_redo<<<std::min<uint32_t>(b.single_max, uint32_t(b.sms) * 2), RW + 32,
+                         size_t(b.kp) * 8, st>>>(a);
+        count_launch();
+    }
     if (b.d < 1 || b.d > 64 || shape < 0 || shape >= batched_shapes()) return cudaErrorInvalidValue;
     if (b.d <= 32) return launch_dp<32>(a, shape, b.sms, st);
     return launch_dp<64>(a, shape, b.sms, st);

@@ -19,8 +19,14 @@
 // again).  Cosine searches read per-row |x|^2 from a scratch array computed
 // once (same summation order, so the values equal the reference's per-pair
 // dot(b, b)).
+//
+// This full search is the form for d > 62, fewer than 16 points per
+// neighbour, and callers without a workspace; otherwise the tensor-core filter
+// (filter.cu) answers almost every query with the same bits, and k_redo_dist and
+// k_redo_replay take those it leaves.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -89,24 +95,96 @@ __device__ __forceinline__ void heap_push_up(float* hd, uint32_t* hi, int len, f
         }
     }
 }
+// Both children are read at once and the new entry is written where it ends
+// (the reference swaps it down level by level; the result is the same).
 __device__ __forceinline__ void heap_replace_down(float* hd, uint32_t* hi, int len, float d,
                                                   uint32_t j) {
-    hd[0] = d;
-    hi[0] = j;
     int p = 0;
     for (;;) {
         const int l = 2 * p + 1, r = 2 * p + 2;
+        const float dl = l < len ? hd[l] : d, dr = r < len ? hd[r] : d;
         int m = p;
-        if (l < len && hd[l] > hd[m]) m = l;
-        if (r < len && hd[r] > hd[m]) m = r;
+        float dm = d;
+        if (dl > dm) {
+            m = l;
+            dm = dl;
+        }
+        if (dr > dm) {
+            m = r;
+            dm = dr;
+        }
         if (m == p) break;
-        const float tv = hd[p];
-        hd[p] = hd[m];
-        hd[m] = tv;
-        const uint32_t ti = hi[p];
+        hd[p] = dm;
         hi[p] = hi[m];
-        hi[m] = ti;
         p = m;
+    }
+    hd[p] = d;
+    hi[p] = j;
+}
+
+// The search's distance of rows a and b (16-byte aligned, zero padded); for the
+// cosine metric an and bn are their |x|^2.
+template <int D>
+__device__ __forceinline__ float exact_dist(const float* __restrict__ a,
+                                            const float* __restrict__ b, int d, int cosine,
+                                            float an, float bn) {
+    if (!cosine) return sq_dist_exact_t<D>(a, b, d);
+    const float dt = dot_exact_t<D>(a, b, d);
+    const float den = __fmul_rn(__fsqrt_rn(an), __fsqrt_rn(bn));
+    return den > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(dt, den)) : 1.0f;
+}
+
+// One warp takes the distances dd of candidates j0 + lane (cnt of them) into
+// its heap, as the reference's sequential scan does.
+__device__ __forceinline__ void replay_tile(float* hd, uint32_t* hi, int& hlen, int kws, float dd,
+                                            uint64_t j0, uint32_t cnt, int lane) {
+    uint32_t pending = cnt == 32 ? FULL : ((1u << cnt) - 1u);
+    // while the heap is short, every candidate is pushed in order
+    while (pending && hlen < kws) {
+        const int l = __ffs(pending) - 1;
+        pending &= pending - 1;
+        const float dl = __shfl_sync(FULL, dd, l);
+        if (lane == 0) heap_push_up(hd, hi, hlen, dl, uint32_t(j0 + l));
+        ++hlen;
+        __syncwarp();
+    }
+    // then the first remaining lane that beats the current root, in order
+    while (pending) {
+        const float root = hd[0];
+        const uint32_t m = __ballot_sync(FULL, ((pending >> lane) & 1u) && dd < root);
+        if (!m) break;
+        const int l = __ffs(m) - 1;
+        pending &= ~((l == 31) ? FULL : ((2u << l) - 1u));
+        const float dl = __shfl_sync(FULL, dd, l);
+        if (lane == 0) heap_replace_down(hd, hi, hlen, dl, uint32_t(j0 + l));
+        __syncwarp();
+    }
+}
+
+// A warp's finished heap as the query's output row: stable ascending sort
+// (insertion), sqrt for Euclidean, the closest entry dropped.
+__device__ __forceinline__ void write_row(float* hd, uint32_t* hi, int hlen, int kws, uint64_t q,
+                                          int cosine, int lane, uint32_t* __restrict__ out_idx,
+                                          float* __restrict__ out_dist) {
+    if (lane == 0) {
+        for (int a = 1; a < hlen; ++a) {
+            const float x = hd[a];
+            const uint32_t y = hi[a];
+            int b = a - 1;
+            while (b >= 0 && hd[b] > x) {
+                hd[b + 1] = hd[b];
+                hi[b + 1] = hi[b];
+                --b;
+            }
+            hd[b + 1] = x;
+            hi[b + 1] = y;
+        }
+    }
+    __syncwarp();
+    const uint64_t per = uint64_t(kws - 1);
+    for (int t = 1 + lane; t < hlen; t += 32) {
+        out_idx[q * per + (t - 1)] = hi[t];
+        out_dist[q * per + (t - 1)] = cosine ? hd[t] : __fsqrt_rn(hd[t]);
     }
 }
 
@@ -138,59 +216,182 @@ __global__ void __launch_bounds__(EW * 32) k_exact_knn(const float* __restrict__
         __syncthreads();
         if (!qv) continue;
         float dd = 0.0f;
-        if (uint32_t(lane) < cnt) {
-            const float* cr = st + lane * dp;
-            if (!cosine) {
-                dd = sq_dist_exact_t<D>(qr, cr, d);
-            } else {
-                const float dt = dot_exact_t<D>(qr, cr, d);
-                const float den = __fmul_rn(__fsqrt_rn(qn), __fsqrt_rn(norms[j0 + lane]));
-                dd = den > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(dt, den)) : 1.0f;
-            }
-        }
-        uint32_t pending = cnt == 32 ? FULL : ((1u << cnt) - 1u);
-        // while the heap is short, every candidate is pushed in order
-        while (pending && hlen < kws) {
-            const int l = __ffs(pending) - 1;
-            pending &= pending - 1;
-            const float dl = __shfl_sync(FULL, dd, l);
-            if (lane == 0) heap_push_up(hd, hi, hlen, dl, uint32_t(j0 + l));
-            ++hlen;
-            __syncwarp();
-        }
-        // then the first remaining lane that beats the current root, in order
-        while (pending) {
-            const float root = hd[0];
-            const uint32_t m = __ballot_sync(FULL, ((pending >> lane) & 1u) && dd < root);
-            if (!m) break;
-            const int l = __ffs(m) - 1;
-            pending &= ~((l == 31) ? FULL : ((2u << l) - 1u));
-            const float dl = __shfl_sync(FULL, dd, l);
-            if (lane == 0) heap_replace_down(hd, hi, hlen, dl, uint32_t(j0 + l));
-            __syncwarp();
+        if (uint32_t(lane) < cnt)
+            dd = exact_dist<D>(qr, st + lane * dp, d, cosine, qn, cosine ? norms[j0 + lane] : 0.0f);
+        replay_tile(hd, hi, hlen, kws, dd, j0, cnt, lane);
+    }
+    if (qv) write_row(hd, hi, hlen, kws, q, cosine, lane, out_idx, out_dist);
+}
+
+// Single queries (those the filter leaves: equal distances among the k + 1
+// nearest, whose order is the heap's), in two steps: k_redo_dist evaluates all
+// their distances, and k_redo_replay walks them as the sequential scan does, a
+// warp per query.  A CTA per query that did both waited for row loads between
+// barriers (346 us for 17 queries at 20,000 x 50, 4.6 ms for 2,762 at 60,013 x
+// 30 cosine).  The distance buffer holds redo_cap queries; k_redo_rest takes
+// those past them.
+constexpr int RQ = 4;     // queries per CTA of k_redo_dist
+constexpr int RD = 256;   // candidates (= threads) per CTA
+
+// dist[u * ld + j] of RQ queries (their rows in sq, dimension-major) and row j;
+// rows are column-major, so every load is one coalesced line.
+template <int D>
+__device__ __forceinline__ void redo_dist4(const float* __restrict__ Xt, uint32_t n, int d_,
+                                           int cosine, const float* __restrict__ norms,
+                                           const float (*sq)[RQ], const float* qn, uint32_t j,
+                                           uint32_t ld, float* __restrict__ dist) {
+    const int d = D > 0 ? D : d_, full = d >> 3;
+    const float* col = Xt + j;
+    float acc[RQ][8], tail[RQ];
+#pragma unroll
+    for (int u = 0; u < RQ; ++u) {
+        tail[u] = 0.0f;
+#pragma unroll
+        for (int l = 0; l < 8; ++l) acc[u][l] = 0.0f;
+    }
+    auto term = [&](float a, float x, float y) {
+        const float t = cosine ? x : __fsub_rn(x, y);
+        return __fadd_rn(a, __fmul_rn(t, cosine ? y : t));
+    };
+#pragma unroll 2
+    for (int c = 0; c < full; ++c) {
+        float y[8];
+#pragma unroll
+        for (int l = 0; l < 8; ++l) y[l] = col[size_t(8 * c + l) * n];
+#pragma unroll
+        for (int l = 0; l < 8; ++l) {
+            const float4 x = *reinterpret_cast<const float4*>(sq[8 * c + l]);
+            acc[0][l] = term(acc[0][l], x.x, y[l]);
+            acc[1][l] = term(acc[1][l], x.y, y[l]);
+            acc[2][l] = term(acc[2][l], x.z, y[l]);
+            acc[3][l] = term(acc[3][l], x.w, y[l]);
         }
     }
-    if (!qv) return;
-    // stable ascending sort (insertion), sqrt for Euclidean, drop the closest
-    if (lane == 0) {
-        for (int a = 1; a < hlen; ++a) {
-            const float x = hd[a];
-            const uint32_t y = hi[a];
-            int b = a - 1;
-            while (b >= 0 && hd[b] > x) {
-                hd[b + 1] = hd[b];
-                hi[b + 1] = hi[b];
-                --b;
+    for (int c = 8 * full; c < d; ++c) {
+        const float y = col[size_t(c) * n];
+#pragma unroll
+        for (int u = 0; u < RQ; ++u) tail[u] = term(tail[u], sq[c][u], y);
+    }
+#pragma unroll
+    for (int u = 0; u < RQ; ++u) {
+        const float* A = acc[u];
+        float r = __fadd_rn(
+            __fadd_rn(__fadd_rn(__fadd_rn(A[0], A[4]), __fadd_rn(A[1], A[5])),
+                      __fadd_rn(__fadd_rn(A[2], A[6]), __fadd_rn(A[3], A[7]))),
+            tail[u]);
+        if (cosine) {
+            const float den = __fmul_rn(__fsqrt_rn(qn[u]), __fsqrt_rn(norms[j]));
+            r = den > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(r, den)) : 1.0f;
+        }
+        dist[size_t(u) * ld + j] = r;
+    }
+}
+
+// The rows of queries [i0, i0 + RQ) of the list (the last one repeated past its
+// end).
+__device__ __forceinline__ void redo_queries(const float* __restrict__ Xt, uint32_t n, int d,
+                                             int cosine, const float* __restrict__ norms,
+                                             const uint32_t* __restrict__ list, uint32_t nq,
+                                             uint32_t i0, float (*sq)[RQ], float* qn) {
+    for (int t = threadIdx.x; t < d * RQ; t += blockDim.x)
+        sq[t / RQ][t % RQ] = Xt[size_t(t / RQ) * n + list[min(i0 + uint32_t(t % RQ), nq - 1)]];
+    if (threadIdx.x < RQ)
+        qn[threadIdx.x] = cosine ? norms[list[min(i0 + threadIdx.x, nq - 1)]] : 0.0f;
+}
+
+// One warp: the sequential scan over a query's distances (512 in flight, 128
+// per vote), then its output row.
+__device__ __forceinline__ void redo_replay(const float* __restrict__ row, uint32_t n, int kws,
+                                            int cosine, uint32_t q, float* hd, uint32_t* hi,
+                                            uint32_t* __restrict__ out_idx,
+                                            float* __restrict__ out_dist) {
+    const int lane = threadIdx.x & 31;
+    int hlen = 0;
+    for (uint32_t j0 = 0; j0 < n; j0 += 512) {
+        float dd[16];
+#pragma unroll
+        for (int g = 0; g < 16; ++g) {
+            const uint32_t j = j0 + 32 * g + lane;
+            dd[g] = j < n ? row[j] : __int_as_float(0x7f800000);
+        }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            bool hit = hlen < kws;
+#pragma unroll
+            for (int g = 4 * v; g < 4 * v + 4; ++g) hit |= hlen == kws && dd[g] < hd[0];
+            if (!__any_sync(FULL, hit)) continue;
+#pragma unroll
+            for (int g = 4 * v; g < 4 * v + 4; ++g) {
+                const uint32_t jg = j0 + 32 * g;
+                if (jg < n)
+                    replay_tile(hd, hi, hlen, kws, dd[g], jg, n - jg < 32 ? n - jg : 32, lane);
             }
-            hd[b + 1] = x;
-            hi[b + 1] = y;
         }
     }
+    write_row(hd, hi, hlen, kws, q, cosine, lane, out_idx, out_dist);
     __syncwarp();
-    const uint64_t per = uint64_t(kws - 1);
-    for (int t = 1 + lane; t < hlen; t += 32) {
-        out_idx[q * per + (t - 1)] = hi[t];
-        out_dist[q * per + (t - 1)] = cosine ? hd[t] : __fsqrt_rn(hd[t]);
+}
+
+// The first cap queries of the list: distances over the whole grid ...
+template <int D>
+__global__ void __launch_bounds__(RD) k_redo_dist(const float* __restrict__ Xt, uint32_t n, int d,
+                                                  int cosine, const float* __restrict__ norms,
+                                                  const uint32_t* __restrict__ list,
+                                                  const uint32_t* __restrict__ list_n,
+                                                  uint32_t cap, uint32_t ld,
+                                                  float* __restrict__ dist) {
+    __shared__ __align__(16) float sq[64][RQ];
+    __shared__ float qn[RQ];
+    const uint32_t nq = min(*list_n, cap), j = blockIdx.x * RD + threadIdx.x;
+    for (uint32_t i0 = blockIdx.y * RQ; i0 < nq; i0 += gridDim.y * RQ) {
+        __syncthreads();
+        redo_queries(Xt, n, d, cosine, norms, list, nq, i0, sq, qn);
+        __syncthreads();
+        if (j < n)
+            redo_dist4<D>(Xt, n, d, cosine, norms, sq, qn, j, ld, dist + size_t(i0) * ld);
+    }
+}
+// ... and their scans, a warp each.
+__global__ void __launch_bounds__(32) k_redo_replay(const float* __restrict__ dist, uint32_t n,
+                                                    uint32_t ld, int kws, int cosine,
+                                                    const uint32_t* __restrict__ list,
+                                                    const uint32_t* __restrict__ list_n,
+                                                    uint32_t cap, uint32_t* __restrict__ out_idx,
+                                                    float* __restrict__ out_dist) {
+    __shared__ float hd[EXACT_MAX_K];
+    __shared__ uint32_t hi[EXACT_MAX_K];
+    const uint32_t nq = min(*list_n, cap);
+    for (uint32_t i = blockIdx.x; i < nq; i += gridDim.x)
+        redo_replay(dist + size_t(i) * ld, n, kws, cosine, list[i], hd, hi, out_idx, out_dist);
+}
+// The queries past the first cap (inputs full of ties): RQ per CTA at a time,
+// their distances in the CTA's own rows of the buffer.
+template <int D>
+__global__ void __launch_bounds__(RD) k_redo_rest(const float* __restrict__ Xt, uint32_t n, int d,
+                                                  int kws, int cosine,
+                                                  const float* __restrict__ norms,
+                                                  const uint32_t* __restrict__ list,
+                                                  const uint32_t* __restrict__ list_n,
+                                                  uint32_t cap, uint32_t ld,
+                                                  float* __restrict__ dist,
+                                                  uint32_t* __restrict__ out_idx,
+                                                  float* __restrict__ out_dist) {
+    __shared__ __align__(16) float sq[64][RQ];
+    __shared__ float qn[RQ];
+    __shared__ float hd[RQ][EXACT_MAX_K];
+    __shared__ uint32_t hi[RQ][EXACT_MAX_K];
+    const uint32_t nq = *list_n, w = threadIdx.x >> 5;
+    float* mine = dist + size_t(blockIdx.x) * RQ * ld;
+    for (uint32_t i0 = cap + blockIdx.x * RQ; i0 < nq; i0 += gridDim.x * RQ) {
+        __syncthreads();
+        redo_queries(Xt, n, d, cosine, norms, list, nq, i0, sq, qn);
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < n; j += RD)
+            redo_dist4<D>(Xt, n, d, cosine, norms, sq, qn, j, ld, mine);
+        __syncthreads();
+        if (w < uint32_t(RQ) && i0 + w < nq)
+            redo_replay(mine + size_t(w) * ld, n, kws, cosine, list[i0 + w], hd[w], hi[w], out_idx,
+                        out_dist);
     }
 }
 
@@ -201,15 +402,34 @@ __global__ void k_exact_indptr(uint32_t* __restrict__ indptr, uint64_t n, uint32
 
 template <int D>
 cudaError_t launch_d(const float* X, uint64_t n, int d, int kws, int cosine, float* norms,
-                     uint32_t* indptr, uint32_t* indices, float* dists, cudaStream_t st) {
+                     uint32_t* indptr, uint32_t* indices, float* dists, cudaStream_t st,
+                     const ExactFilter* filter) {
     const int dp = (d + 3) / 4 * 4;
     if (cosine) {
         k_row_dots<<<uint32_t((n + 255) / 256), 256, 0, st>>>(X, n, d, norms);
         count_launch();
     }
-    k_exact_knn<D><<<uint32_t((n + EW - 1) / EW), EW * 32, exact_knn_smem(d, kws), st>>>(
-        X, uint32_t(n), d, dp, kws, cosine, norms, indices, dists);
-    count_launch();
+    if (filter) {
+        cudaError_t e = cudaMemsetAsync(filter->redo_n, 0, 4, st);
+        if (e == cudaSuccess) e = filter->run(st);
+        if (e != cudaSuccess) return e;
+        const uint32_t cap = filter->redo_cap, ld = filter->redo_ld;
+        const dim3 grid(uint32_t((n + RD - 1) / RD), 16);
+        k_redo_dist<D><<<grid, RD, 0, st>>>(filter->Xt, uint32_t(n), d, cosine, norms, filter->redo,
+                                            filter->redo_n, cap, ld, filter->redo_dist);
+        k_redo_replay<<<148 * 16, 32, 0, st>>>(filter->redo_dist, uint32_t(n), ld, kws, cosine,
+                                              filter->redo, filter->redo_n, cap, indices, dists);
+        k_redo_rest<D><<<std::min<uint32_t>(cap / RQ, 148 * 4), RD, 0, st>>>(
+            filter->Xt, uint32_t(n), d, kws, cosine, norms, filter->redo, filter->redo_n, cap, ld,
+            filter->redo_dist, indices, dists);
+        count_launch();
+        count_launch();
+        count_launch();
+    } else {
+        k_exact_knn<D><<<uint32_t((n + EW - 1) / EW), EW * 32, exact_knn_smem(d, kws), st>>>(
+            X, uint32_t(n), d, dp, kws, cosine, norms, indices, dists);
+        count_launch();
+    }
     k_exact_indptr<<<uint32_t((n + 256) / 256), 256, 0, st>>>(indptr, n, uint32_t(kws - 1));
     count_launch();
     return cudaGetLastError();
@@ -236,12 +456,13 @@ cudaError_t exact_knn_prepare() {
 
 cudaError_t launch_exact_knn(const float* X, uint64_t n, int d, int kws, int cosine,
                              float* norms, uint32_t* indptr, uint32_t* indices, float* dists,
-                             cudaStream_t st) {
+                             cudaStream_t st, const ExactFilter* filter) {
     if (n == 0 || n > 0xFFFFFFFEull || d < 1 || d > EXACT_MAX_DIM || kws < 1 ||
         kws > EXACT_MAX_K)
         return cudaErrorInvalidValue;
-    if (d == 50) return launch_d<50>(X, n, d, kws, cosine, norms, indptr, indices, dists, st);
-    return launch_d<0>(X, n, d, kws, cosine, norms, indptr, indices, dists, st);
+    if (d == 50)
+        return launch_d<50>(X, n, d, kws, cosine, norms, indptr, indices, dists, st, filter);
+    return launch_d<0>(X, n, d, kws, cosine, norms, indptr, indices, dists, st, filter);
 }
 
 }  // namespace pq

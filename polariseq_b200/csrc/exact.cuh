@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <functional>
+
 namespace pq {
 
 constexpr int EXACT_MAX_DIM = 512;  // n_dim limit of the staged-tile kernel
@@ -17,8 +19,18 @@ cudaError_t exact_knn_prepare();
 // Enqueues the search on `st`: indptr (n+1), indices / dists (n * (kws-1)).
 // `norms` (n floats) is scratch for the cosine metric (unused for Euclidean);
 // every element the kernels read is written first in the same launch sequence.
+// With `filter`, its prepared steps run first (after the norms) and the search
+// takes the queries they leave in `redo`.
+struct ExactFilter {
+    std::function<cudaError_t(cudaStream_t)> run;
+    uint32_t* redo;    // device: query rows
+    uint32_t* redo_n;  // device: their number
+    const float* Xt;   // device: the rows column-major [d][n], written by `run`
+    float* redo_dist;  // device: distances of redo_cap queries, redo_ld apart
+    uint32_t redo_cap, redo_ld;
+};
 cudaError_t launch_exact_knn(const float* X, uint64_t n, int d, int kws, int cosine,
                              float* norms, uint32_t* indptr, uint32_t* indices, float* dists,
-                             cudaStream_t st);
+                             cudaStream_t st, const ExactFilter* filter = nullptr);
 
 }  // namespace pq
