@@ -469,7 +469,7 @@ uint64_t build_plain(pq_ctx* c, const float* data, bool data_on_host, uint64_t n
            "upload roots");
         KGScope kg(c, PQ_KG_SEQTREE);
         uint32_t n_big = 0;
-        while (n_big < roots.size() && n_big < 148 && roots[n_big].size > 65536) ++n_big;
+        while (n_big < roots.size() && n_big < 148 && roots[n_big].size > SEQ_BIG_MIN) ++n_big;
         if (fa.trace) {
             uint64_t r0 = roots.empty() ? 0 : roots[0].size;
             ck(cudaMemcpyAsync(fa.trace + SEQ_T_ROOT0, &r0, 8, cudaMemcpyHostToDevice, st), "tr");
@@ -495,34 +495,24 @@ uint64_t build_plain(pq_ctx* c, const float* data, bool data_on_host, uint64_t n
                      T, (unsigned long long)R.leaf_size, S.ms_forest, roots.size(), h[SEQ_T_ROOT0]);
         std::fprintf(stderr,
                      "[nndescent]   subtrees: global nodes %llu (points %llu), staged subtrees "
-                     "%llu (nodes %llu), tie nodes %llu, random splits %llu\n",
-                     h[0], h[1], h[2], h[3], h[4], h[5]);
+                     "%llu (CTA splits %llu, warp splits %llu), tie nodes %llu, random splits %llu\n",
+                     h[SEQ_T_GLOBAL_NODES], h[SEQ_T_GLOBAL_POINTS], h[SEQ_T_STAGED_TREES],
+                     h[SEQ_T_MID_NODES], h[SEQ_T_STAGED_NODES], h[SEQ_T_TIES],
+                     h[SEQ_T_DEGENERATE]);
         std::fprintf(stderr,
                      "[nndescent]   largest subtree cycles: draw %llu margin %llu partition %llu "
-                     "staged %llu total %llu\n",
-                     h[6], h[7], h[8], h[9], h[10]);
-        std::fprintf(stderr,
-                     "[nndescent]   largest subtree: global nodes %llu, CTA-staged nodes %llu, "
-                     "staged subtrees %llu (nodes %llu, warp cycles %llu); CTA-staged subtrees "
-                     "%llu (nodes %llu) in all\n",
-                     h[SEQ_T_R0_GNODES], h[SEQ_T_R0_MNODES], h[SEQ_T_R0_STAGED],
-                     h[SEQ_T_R0_SNODES], h[SEQ_T_R0_CYC_WARP], h[SEQ_T_MID_TREES],
-                     h[SEQ_T_MID_NODES]);
-        std::fprintf(stderr,
-                     "[nndescent]   largest subtree, warp splits: leaf pops %llu draws %llu "
-                     "margins %llu partition %llu; CTA splits: staging %llu draws %llu margins "
-                     "%llu partition %llu cycles\n",
-                     h[SEQ_T_W_LEAF], h[SEQ_T_W_DRAW], h[SEQ_T_W_MARGIN], h[SEQ_T_W_PART],
-                     h[SEQ_T_M_STAGE], h[SEQ_T_M_DRAW], h[SEQ_T_M_MARGIN], h[SEQ_T_M_PART]);
+                     "staged %llu (warp splits %llu) total %llu\n",
+                     h[SEQ_T_CYC_DRAW], h[SEQ_T_CYC_MARGIN], h[SEQ_T_CYC_PART],
+                     h[SEQ_T_CYC_STAGED], h[SEQ_T_R0_CYC_WARP], h[SEQ_T_CYC_TOTAL]);
         // timeline of the two subtree kernels (globaltimer): each large root's
         // CTA against the span of the 128-thread kernel
         uint32_t nb = 0;
-        while (nb < roots.size() && nb < 148 && roots[nb].size > 65536) ++nb;
+        while (nb < roots.size() && nb < 148 && roots[nb].size > SEQ_BIG_MIN) ++nb;
         unsigned long long t0 = ~h[SEQ_T_SMALL_T0], t1s = h[SEQ_T_SMALL_T1];
         for (uint32_t b = 0; b < nb && b < uint32_t(SEQ_T_BIG_N); ++b)
             t0 = std::min(t0, h[SEQ_T_BIG + 2 * b]);
         std::fprintf(stderr,
-                     "[nndescent]   subtree timeline: %u roots above 65536 points, %zu below; "
+                     "[nndescent]   subtree timeline: %u large roots, %zu others; "
                      "128-thread kernel ends at %.2f ms\n",
                      nb, roots.size() - nb, (t1s - t0) * 1e-6);
         for (uint32_t b = 0; b < nb && b < uint32_t(SEQ_T_BIG_N); ++b) {

@@ -48,37 +48,28 @@ enum {
     SEQ_T_GLOBAL_NODES = 0,   // nodes split in global mode
     SEQ_T_GLOBAL_POINTS = 1,  // margins evaluated in global mode
     SEQ_T_STAGED_TREES = 2,   // staged subtrees
-    SEQ_T_STAGED_NODES = 3,   // nodes split in staged subtrees
+    SEQ_T_STAGED_NODES = 3,   // their nodes split by warp 0
     SEQ_T_TIES = 4,           // nodes with tie draws
     SEQ_T_DEGENERATE = 5,     // random splits
-    SEQ_T_CYC_DRAW = 6,       // block 0 cycles: draws + hyperplane rows
-    SEQ_T_CYC_MARGIN = 7,     // block 0 cycles: global-mode margins
-    SEQ_T_CYC_PART = 8,       // block 0 cycles: global-mode partition
-    SEQ_T_CYC_STAGED = 9,     // block 0 cycles: staged subtrees
-    SEQ_T_CYC_TOTAL = 10,     // block 0 cycles: whole kernel
-    SEQ_T_ROOT0 = 11,         // block 0 root size
-    SEQ_T_R0_STAGED = 12,     // block 0: staged subtrees
-    SEQ_T_R0_SNODES = 13,     // block 0: nodes split in staged subtrees
-    SEQ_T_R0_GNODES = 14,     // block 0: nodes split in global mode
-    SEQ_T_R0_CYC_WARP = 15,   // block 0 cycles: warp 0's splits of staged subtrees
-    SEQ_T_MID_TREES = 16,     // staged subtrees of up to 512 points (512-thread CTAs)
-    SEQ_T_MID_NODES = 17,     // their nodes split by the whole CTA
-    SEQ_T_R0_MNODES = 18,     // block 0: the same
-    SEQ_T_W_LEAF = 20,        // block 0 cycles, warp 0's staged splits: leaf pops
-    SEQ_T_W_DRAW = 21,        //   draws
-    SEQ_T_W_MARGIN = 22,      //   normal, offset, margins, sides
-    SEQ_T_W_PART = 23,        //   partition and pushes
-    SEQ_T_M_DRAW = 24,        // block 0 cycles, CTA-staged splits: draws
-    SEQ_T_M_MARGIN = 25,      //   normal, offset, margins, sides
-    SEQ_T_M_PART = 26,        //   partition
-    SEQ_T_M_STAGE = 27,       //   staging ids and rows
-    SEQ_T_SMALL_T0 = 28,      // 128-thread CTAs: earliest start (globaltimer ns)
-    SEQ_T_SMALL_T1 = 29,      //   latest end
-    SEQ_T_BIG = 32,           // 512-thread CTAs: start and end (globaltimer ns) of each of
-                              // the first SEQ_T_BIG_N, slots SEQ_T_BIG + 2 * block (+ 1)
+    SEQ_T_CYC_DRAW = 6,       // largest subtree, cycles: global-mode draws and hyperplanes
+    SEQ_T_CYC_MARGIN = 7,     //   global-mode margins
+    SEQ_T_CYC_PART = 8,       //   global-mode partition
+    SEQ_T_CYC_STAGED = 9,     //   staged subtrees
+    SEQ_T_CYC_TOTAL = 10,     //   the whole subtree
+    SEQ_T_ROOT0 = 11,         // its size
+    SEQ_T_R0_CYC_WARP = 12,   //   cycles of warp 0's splits
+    SEQ_T_MID_NODES = 13,     // staged nodes split by the whole CTA
+    SEQ_T_SMALL_T0 = 14,      // 128-thread CTAs: earliest start (globaltimer ns)
+    SEQ_T_SMALL_T1 = 15,      //   latest end
+    SEQ_T_BIG = 16,           // the largest subtrees' CTAs: start and end (globaltimer ns) of
+                              // each of the first SEQ_T_BIG_N, slots SEQ_T_BIG + 2 * block (+ 1)
     SEQ_T_BIG_N = 148,
     SEQ_TRACE_N = SEQ_T_BIG + 2 * SEQ_T_BIG_N
 };
+
+// The largest subtrees, at most one per SM, take the wider CTA when they hold
+// more points than this.
+constexpr uint32_t SEQ_BIG_MIN = 2048;
 
 constexpr int FOREST_CHUNK = 2048;
 
