@@ -248,6 +248,13 @@ int pq_mlp_grad(pq_ctx* ctx, uint64_t n_dim, const float* params, const float* X
                 const uint32_t* tb, const float* tw, uint32_t T, float* grad_out,
                 float* loss_out, float* logits_out);
 
+/* Copies between HOST arrays and device memory through the context: large
+ * pageable arrays go through its pinned ring with several host threads (the
+ * host-buffer entry points above do the same).  Ordered after `stream` (a
+ * cudaStream_t, may be null); complete on return. */
+int pq_copy_to_device(pq_ctx* ctx, void* d_dst, const void* src, uint64_t bytes, void* stream);
+int pq_copy_to_host(pq_ctx* ctx, void* dst, const void* d_src, uint64_t bytes, void* stream);
+
 /* Flags of pq_knn_batched_into_device. */
 enum { PQ_BATCH_AUTOTUNE = 1, PQ_BATCH_GRAPH = 2 };
 

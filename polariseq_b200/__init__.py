@@ -219,9 +219,9 @@ class Context:
         ix = np.ascontiguousarray(indices, np.uint32)
         dx = np.ascontiguousarray(data, np.float32)
         cap = max(2 * int(ip[n_obs]), 1)
-        oip = np.zeros(n_obs + 1, np.uint32)
-        oix = np.zeros(cap, np.uint32)
-        ow = np.zeros(cap, np.float32)
+        oip = np.empty(n_obs + 1, np.uint32)
+        oix = np.empty(cap, np.uint32)  # (entries past the result are never touched)
+        ow = np.empty(cap, np.float32)
         nnz = C.c_uint64(0)
         with self._lock:
             rc = _lib.load().pq_fuzzy_connectivities(
@@ -229,7 +229,25 @@ class Context:
                 oix.ctypes.data, ow.ctypes.data, cap, C.byref(nnz))
             self._check(rc, "fuzzy_connectivities")
         m = int(nnz.value)
-        return {"indptr": oip, "indices": oix[:m].copy(), "data": ow[:m].copy()}
+        return {"indptr": oip, "indices": oix[:m], "data": ow[:m]}
+
+    # -- host copies ---------------------------------------------------------
+    def copy_to_device(self, dst, src: np.ndarray, offset: int = 0, stream=None) -> None:
+        """A contiguous array's bytes into the CUDA tensor `dst`, `offset` bytes
+        in, after what `stream` still does with it."""
+        sp = None if stream is None else C.c_void_p(int(stream))
+        with self._lock:
+            rc = _lib.load().pq_copy_to_device(self._h, dst.data_ptr() + offset, src.ctypes.data,
+                                               src.nbytes, sp)
+            self._check(rc, "copy_to_device")
+
+    def copy_to_host(self, dst: np.ndarray, src, stream=None) -> None:
+        """The first bytes of the CUDA tensor `src` into a contiguous array."""
+        sp = None if stream is None else C.c_void_p(int(stream))
+        with self._lock:
+            rc = _lib.load().pq_copy_to_host(self._h, dst.ctypes.data, src.data_ptr(), dst.nbytes,
+                                             sp)
+            self._check(rc, "copy_to_host")
 
     # -- parity probes (test hooks) ----------------------------------------
     def probe(self, data: np.ndarray, opts: _lib.NndOpts, stop_after: int) -> dict:
@@ -333,9 +351,9 @@ def nndescent_dense(embedding, k, max_iterations=0, seed=0, max_candidates=0, n_
     if out is not None:
         nnz = ctx.nndescent_into(emb, opts, ip, ix, dx)
         return {"nnz": nnz, "n_obs": n_obs}
-    ip = np.zeros(n_obs + 1, np.uint32)
-    ix = np.zeros(cap, np.uint32)
-    dx = np.zeros(cap, np.float32)
+    ip = np.empty(n_obs + 1, np.uint32)
+    ix = np.empty(cap, np.uint32)  # (entries past nnz are cut off below)
+    dx = np.empty(cap, np.float32)
     nnz = ctx.nndescent_into(emb, opts, ip, ix, dx)
     return {"indptr": ip, "indices": ix[:nnz], "data": dx[:nnz], "n_obs": n_obs}
 
@@ -373,13 +391,31 @@ def knn_batched(samples, ks, *, device: int = 0, autotune: bool = False, graph: 
     ks = np.asarray(ks, np.uint32)
     total = int(np.sum(sizes * ks.astype(np.uint64)))
     dev = torch.device("cuda", device)
-    x = torch.from_numpy(np.concatenate(arrs, 0)).to(dev)
-    oi = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-    od = torch.empty(max(total, 1), dtype=torch.float32, device=dev)
-    default_context(device).knn_batched_device(x, offsets, ks, oi, od, autotune=autotune,
-                                               graph=graph)
-    oi = oi.cpu().numpy().view(np.uint32)
-    od = od.cpu().numpy()
+    if any(a.ndim != 2 or a.shape[1] != d for a in arrs):
+        raise ValueError("knn_batched: the samples must be 2-D with the same number of columns")
+    ctx = default_context(device)
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    x = torch.empty((int(offsets[-1]), d), dtype=torch.float32, device=dev)
+    # small samples are joined first: a copy of its own costs each a round trip
+    small, at = [], 0
+    for i, a in enumerate(arrs):
+        if a.nbytes < (1 << 20):
+            small.append(a)
+        if small and (a.nbytes >= (1 << 20) or i + 1 == len(arrs)):
+            blk = np.concatenate(small, 0)
+            ctx.copy_to_device(x, blk, at, stream)
+            at += blk.nbytes
+            small = []
+        if a.nbytes >= (1 << 20):
+            ctx.copy_to_device(x, a, at, stream)
+            at += a.nbytes
+    doi = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
+    dod = torch.empty(max(total, 1), dtype=torch.float32, device=dev)
+    ctx.knn_batched_device(x, offsets, ks, doi, dod, autotune=autotune, graph=graph,
+                           stream=stream)
+    oi, od = np.empty(max(total, 1), np.uint32), np.empty(max(total, 1), np.float32)
+    ctx.copy_to_host(oi, doi, stream)
+    ctx.copy_to_host(od, dod, stream)
     out, o = [], 0
     for a, k in zip(arrs, ks):
         m = a.shape[0] * int(k)
@@ -517,9 +553,9 @@ def neighbors_dense(embedding, n_neighbors, metric, *, device: int = 0) -> dict:
     n_obs = emb.shape[0]
     kws = min(int(n_neighbors), n_obs)
     nnz_cap = max(n_obs * max(kws - 1, 0), 1)
-    ip = np.zeros(n_obs + 1, np.uint32)
-    ix = np.zeros(nnz_cap, np.uint32)
-    dx = np.zeros(nnz_cap, np.float32)
+    ip = np.empty(n_obs + 1, np.uint32)
+    ix = np.empty(nnz_cap, np.uint32)
+    dx = np.empty(nnz_cap, np.float32)
     nnz = default_context(device).neighbors_into(emb, int(n_neighbors), m, ip, ix, dx)
     return {"indptr": ip, "indices": ix[:nnz], "data": dx[:nnz], "n_obs": n_obs}
 
@@ -540,8 +576,8 @@ def nndescent(data: np.ndarray, k: int = 15, *, max_candidates=0, max_iterations
     opts = _opts(k, max_iterations, seed, max_candidates, n_trees, delta, leaf_size, gather_max,
                  mode=MODES[mode], init=INITS[init], probes=probes, refine_rounds=refine_rounds)
     cap = n_obs * effective_k(n_obs, k)
-    ip = np.zeros(n_obs + 1, np.uint32)
-    ix = np.zeros(cap, np.uint32)
-    dx = np.zeros(cap, np.float32)
+    ip = np.empty(n_obs + 1, np.uint32)
+    ix = np.empty(cap, np.uint32)
+    dx = np.empty(cap, np.float32)
     nnz = default_context(device).nndescent_into(emb, opts, ip, ix, dx)
     return {"indptr": ip, "indices": ix[:nnz], "data": dx[:nnz], "n_obs": n_obs}

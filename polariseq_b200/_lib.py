@@ -24,6 +24,7 @@ EXPORTS = (
     "pq_ctx_last_error", "pq_ctx_stats", "pq_nndescent_into", "pq_nndescent_into_device",
     "pq_nndescent_probe", "pq_debug_tree", "pq_ctx_set_profiling", "pq_neighbors_into",
     "pq_neighbors_into_device", "pq_neighbors_into_device_noalloc", "pq_knn_batched_into_device",
+    "pq_copy_to_device", "pq_copy_to_host",
     "pq_mlp_params", "pq_mlp_grad", "pq_fuzzy_connectivities", "pq_fuzzy_connectivities_device",
     "pq_ctx_set_test_wait", "pq_scrublet_scores_device",
 )
@@ -149,6 +150,10 @@ def load(build_if_missing: bool = False):
         L.pq_knn_batched_into_device.argtypes = [P, P, U64, C.c_uint32, P, P, P, P, C.c_int32,
                                                   C.POINTER(C.c_int32), P]
         L.pq_knn_batched_into_device.restype = C.c_int
+        L.pq_copy_to_device.argtypes = [P, P, P, U64, P]
+        L.pq_copy_to_device.restype = C.c_int
+        L.pq_copy_to_host.argtypes = [P, P, P, U64, P]
+        L.pq_copy_to_host.restype = C.c_int
         L.pq_mlp_params.argtypes = [U64]
         L.pq_mlp_params.restype = U64
         L.pq_mlp_grad.argtypes = [P, U64, P, P, U64, P, P, C.c_uint32, P, P, P]

@@ -134,15 +134,14 @@ float* load_embedding(pq_ctx* c, const float* data, bool on_host, uint32_t n, in
     float* X = c->get<float>("X", size_t(n) * dp);
     const size_t bytes = size_t(n) * d * sizeof(float);
     if (dp == d) {
-        ck(cudaMemcpyAsync(X, data, bytes,
-                           on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, st),
-           "copy embedding");
+        if (on_host) pq::copy_to_device(c, X, data, bytes, st);
+        else ck(cudaMemcpyAsync(X, data, bytes, cudaMemcpyDeviceToDevice, st), "copy embedding");
         return X;
     }
     const float* src = data;
     if (on_host) {  // one contiguous transfer, then the padding on the device
         float* stage = c->get<float>("X_stage", size_t(n) * d);
-        ck(cudaMemcpyAsync(stage, data, bytes, cudaMemcpyHostToDevice, st), "copy embedding");
+        pq::copy_to_device(c, stage, data, bytes, st);
         src = stage;
     }
     k_pad_rows<<<blocks(size_t(n) * dp, 256), 256, 0, st>>>(src, n, d, dp, X);
@@ -157,15 +156,13 @@ float* load_embedding_rows(pq_ctx* c, const float* data, uint32_t n, int d, int 
     if (r1 <= r0) return X;
     const size_t rows = r1 - r0;
     if (dp == d) {
-        ck(cudaMemcpyAsync(X + size_t(r0) * dp, data + size_t(r0) * d, rows * d * sizeof(float),
-                           cudaMemcpyHostToDevice, st),
-           "copy embedding");
+        pq::copy_to_device(c, X + size_t(r0) * dp, data + size_t(r0) * d, rows * d * sizeof(float),
+                           st);
         return X;
     }
     float* stage = c->get<float>("X_stage", size_t(n) * d);
-    ck(cudaMemcpyAsync(stage + size_t(r0) * d, data + size_t(r0) * d, rows * d * sizeof(float),
-                       cudaMemcpyHostToDevice, st),
-       "copy embedding");
+    pq::copy_to_device(c, stage + size_t(r0) * d, data + size_t(r0) * d, rows * d * sizeof(float),
+                       st);
     k_pad_rows<<<blocks(rows * dp, 256), 256, 0, st>>>(stage + size_t(r0) * d, rows, d, dp,
                                                         X + size_t(r0) * dp);
     pq::count_launch();
@@ -872,6 +869,7 @@ void pq_ctx_destroy(pq_ctx* c) {
     if (c->sub) pq_ctx_destroy(c->sub);
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
+    if (c->stage) pq::host_stage_free(c->stage);
     for (auto& kv : c->bufs)
         if (kv.second.p) cudaFree(kv.second.p);
     if (c->d_err) cudaFree(c->d_err);
@@ -928,10 +926,9 @@ int pq_nndescent_into(pq_ctx* c, const float* data, uint64_t n, uint64_t d,
                            ? build_learned_nnd(c, data, true, n, d, *o, dip, dix, ddx)
                            : build_plain(c, data, true, n, d, *o, dip, dix, ddx, nullptr);
         if (!hg.copied) {
-            ck(cudaMemcpyAsync(indptr, dip, (n + 1) * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
-            ck(cudaMemcpyAsync(indices, dix, nnz * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
-            ck(cudaMemcpyAsync(dists, ddx, nnz * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
-            ck(cudaStreamSynchronize(c->stream), "d2h");
+            pq::copy_to_host(c, indptr, dip, (n + 1) * 4, c->stream);
+            pq::copy_to_host(c, indices, dix, nnz * 4, c->stream);
+            pq::copy_to_host(c, dists, ddx, nnz * 4, c->stream);
         }
         *nnz_out = nnz;
         return PQ_OK;
@@ -1027,19 +1024,18 @@ int pq_neighbors_into(pq_ctx* c, const float* data, uint64_t n, uint64_t d,
         uint32_t* dip = c->get<uint32_t>("out_indptr", n + 1);
         uint32_t* dix = c->get<uint32_t>("out_indices", std::max<uint64_t>(nnz, 1));
         float* ddx = c->get<float>("out_dists", std::max<uint64_t>(nnz, 1));
-        ck(cudaMemcpyAsync(X, data, n * d * 4, cudaMemcpyHostToDevice, st), "h2d");
+        pq::copy_to_device(c, X, data, n * d * 4, st);
         ck(pq::exact_knn_prepare(), "exact kNN set-up");
         pq::ExactFilter flt;
         const bool fl = prepare_exact_filter(c, X, n, d, kws, metric, norms, dix, ddx, &flt);
         ck(pq::launch_exact_knn(X, n, int(d), int(kws), metric == PQ_METRIC_COSINE, norms, dip, dix,
                             ddx, st, fl ? &flt : nullptr),
            "exact kNN");
-        ck(cudaMemcpyAsync(indptr, dip, (n + 1) * 4, cudaMemcpyDeviceToHost, st), "d2h");
+        pq::copy_to_host(c, indptr, dip, (n + 1) * 4, st);
         if (nnz) {
-            ck(cudaMemcpyAsync(indices, dix, nnz * 4, cudaMemcpyDeviceToHost, st), "d2h");
-            ck(cudaMemcpyAsync(dists, ddx, nnz * 4, cudaMemcpyDeviceToHost, st), "d2h");
+            pq::copy_to_host(c, indices, dix, nnz * 4, st);
+            pq::copy_to_host(c, dists, ddx, nnz * 4, st);
         }
-        ck(cudaStreamSynchronize(st), "d2h");
         *nnz_out = nnz;
         return PQ_OK;
     });
@@ -1316,6 +1312,38 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
     });
 }
 
+int pq_copy_to_device(pq_ctx* c, void* d_dst, const void* src, uint64_t bytes, void* stream) {
+    if (!c) return PQ_EINVAL;
+    if (bytes == 0) return PQ_OK;
+    if (!d_dst || !src) return fail(c, PQ_EINVAL, "null buffer");
+    return guarded(c, [&]() -> int {
+        // after whatever `stream` still does with the destination
+        cudaEvent_t ev;
+        ck(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
+        ck(cudaEventRecord(ev, static_cast<cudaStream_t>(stream)), "event");
+        ck(cudaStreamWaitEvent(c->stream, ev, 0), "event");
+        cudaEventDestroy(ev);
+        pq::copy_to_device(c, d_dst, src, bytes, c->stream);
+        ck(cudaStreamSynchronize(c->stream), "h2d");
+        return PQ_OK;
+    });
+}
+
+int pq_copy_to_host(pq_ctx* c, void* dst, const void* d_src, uint64_t bytes, void* stream) {
+    if (!c) return PQ_EINVAL;
+    if (bytes == 0) return PQ_OK;
+    if (!dst || !d_src) return fail(c, PQ_EINVAL, "null buffer");
+    return guarded(c, [&]() -> int {
+        cudaEvent_t ev;
+        ck(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
+        ck(cudaEventRecord(ev, static_cast<cudaStream_t>(stream)), "event");
+        ck(cudaStreamWaitEvent(c->stream, ev, 0), "event");
+        cudaEventDestroy(ev);
+        pq::copy_to_host(c, dst, d_src, bytes, c->stream);
+        return PQ_OK;
+    });
+}
+
 uint64_t pq_mlp_params(uint64_t n_dim) { return pq::mlp_params(int(n_dim)); }
 
 int pq_mlp_grad(pq_ctx* c, uint64_t d, const float* params, const float* X, uint64_t rows,
@@ -1403,21 +1431,20 @@ int pq_fuzzy_connectivities(pq_ctx* c, uint64_t n, const uint32_t* indptr,
         uint32_t* oip = c->get<uint32_t>("fz_oip", n + 1);
         uint32_t* oix = c->get<uint32_t>("fz_oix", cap);
         float* ow = c->get<float>("fz_ow", cap);
-        ck(cudaMemcpyAsync(ip, indptr, (n + 1) * 4, cudaMemcpyHostToDevice, st), "h2d");
+        pq::copy_to_device(c, ip, indptr, (n + 1) * 4, st);
         if (nnz) {
-            ck(cudaMemcpyAsync(ix, indices, nnz * 4, cudaMemcpyHostToDevice, st), "h2d");
-            ck(cudaMemcpyAsync(dx, data, nnz * 4, cudaMemcpyHostToDevice, st), "h2d");
+            pq::copy_to_device(c, ix, indices, nnz * 4, st);
+            pq::copy_to_device(c, dx, data, nnz * 4, st);
         }
         uint64_t m = 0;
         const int rc = fuzzy_run(c, n, nnz, ip, ix, dx, oip, oix, ow, cap, &m, st);
         if (rc != PQ_OK) return rc;
         if (m > out_cap) return fail(c, PQ_EINVAL, "the connectivity arrays are too short");
-        ck(cudaMemcpyAsync(out_indptr, oip, (n + 1) * 4, cudaMemcpyDeviceToHost, st), "d2h");
+        pq::copy_to_host(c, out_indptr, oip, (n + 1) * 4, st);
         if (m) {
-            ck(cudaMemcpyAsync(out_indices, oix, m * 4, cudaMemcpyDeviceToHost, st), "d2h");
-            ck(cudaMemcpyAsync(out_weights, ow, m * 4, cudaMemcpyDeviceToHost, st), "d2h");
+            pq::copy_to_host(c, out_indices, oix, m * 4, st);
+            pq::copy_to_host(c, out_weights, ow, m * 4, st);
         }
-        ck(cudaStreamSynchronize(st), "d2h");
         *nnz_out = m;
         return PQ_OK;
     });

@@ -12,6 +12,7 @@
 
 #include "../../include/polariseq_knn.h"
 #include "common.cuh"
+#include "hostcopy.cuh"
 
 namespace pqh {
 
@@ -118,6 +119,7 @@ struct pq_ctx {
     // the learned-init subsample's plain graph is built on this context, kept
     // from build to build (its workspace is not reallocated each time)
     pq_ctx* sub = nullptr;
+    pq::HostStage* stage = nullptr;  // pinned staging of large host copies
 
     template <class T>
     T* get(const std::string& name, size_t count) {
