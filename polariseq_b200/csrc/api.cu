@@ -549,11 +549,16 @@ uint64_t build_plain(pq_ctx* c, const float* data, bool data_on_host, uint64_t n
     {
         uint32_t* leaf_start = fa.tabA;  // reused: the forest scratch is free now
         uint32_t* scanbuf = fa.tabB;
-        void* stemp = c->get<uint8_t>("scan_temp", scan_temp_bytes(n));
         uint64_t* cnts = c->get<uint64_t>("leaf_counts", T);
-        for (uint32_t t = 0; t < T; ++t)
-            launch_leaf_compact(fa.leafflag + size_t(t) * n, n, leaf_start + size_t(t) * n,
-                                scanbuf + size_t(t) * n, stemp, cnts + t, st);
+        // the trees' leaves together stay below 2^32 (a group of trees at a time
+        // beyond that many positions)
+        const uint32_t tg = uint32_t(std::max<uint64_t>(
+            1, std::min<uint64_t>(T, (uint64_t(1) << 32) / std::max<uint32_t>(n, 1) - 1)));
+        void* stemp = c->get<uint8_t>("scan_temp_l", scan_temp_bytes(size_t(tg) * n));
+        for (uint32_t t = 0; t < T; t += tg)
+            launch_leaf_compact(fa.leafflag + size_t(t) * n, std::min(tg, T - t), n,
+                                leaf_start + size_t(t) * n, scanbuf + size_t(t) * n, stemp,
+                                cnts + t, c->d_u64, st);
         std::vector<uint64_t> hc(T);
         ck(cudaMemcpyAsync(hc.data(), cnts, T * sizeof(uint64_t), cudaMemcpyDeviceToHost, st),
            "leaf counts");

@@ -269,15 +269,27 @@ __global__ void k_degenerate(ForestArgs a, PNode* nodes, uint32_t nn) {
     nodes[ni].nL = nd.size / 2;
 }
 
-// Compact leaf starts of one tree: flags (u8) -> u32 -> exclusive scan -> positions.
-__global__ void k_flags_u32(const uint8_t* f, uint32_t n, uint32_t* out) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = f[i];
+// Leaf starts of all trees: flags (u8) -> u32 -> one exclusive scan over the
+// trees' positions -> each tree's positions from its own first leaf.  One pass
+// for all trees instead of five launches per tree (48 trees at 20,000 cells:
+// 240 launches of a few microseconds).
+__global__ void k_flags_u32(const uint8_t* f, size_t tn, uint32_t* out) {
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < tn) out[i] = f[i];
 }
-__global__ void k_leaf_scatter(const uint8_t* f, const uint32_t* pre, uint32_t n,
+__global__ void k_leaf_scatter(const uint8_t* f, const uint32_t* pre, size_t tn, uint32_t n,
                                uint32_t* leaf_start) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && f[i]) leaf_start[pre[i]] = i;
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= tn || !f[i]) return;
+    const size_t t0 = i / n * n;
+    leaf_start[t0 + (pre[i] - pre[t0])] = uint32_t(i - t0);
+}
+__global__ void k_leaf_counts(const uint32_t* pre, const uint64_t* total, uint32_t T, uint32_t n,
+                              uint64_t* counts) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    const uint64_t end = t + 1 < T ? uint64_t(pre[size_t(t + 1) * n]) : *total;
+    counts[t] = end - pre[size_t(t) * n];
 }
 
 // Leaf all-pairs of one tree (nndescent.rs:785-815).  The member at a
@@ -459,12 +471,15 @@ void launch_partition(const ForestArgs& a, PNode* nodes, const uint32_t* chunk_n
 void launch_degenerate(const ForestArgs& a, PNode* nodes, uint32_t nn, cudaStream_t st) {
     k_degenerate<<<(nn + 63) / 64, 64, 0, st>>>(a, nodes, nn); count_launch();
 }
-void launch_leaf_compact(const uint8_t* leafflag_t, uint32_t n, uint32_t* leaf_start,
-                         uint32_t* scan_buf, void* scan_temp, uint64_t* count_dev,
+void launch_leaf_compact(const uint8_t* leafflag, uint32_t T, uint32_t n, uint32_t* leaf_start,
+                         uint32_t* scan_buf, void* scan_temp, uint64_t* counts, uint64_t* total,
                          cudaStream_t st) {
-    k_flags_u32<<<(n + 255) / 256, 256, 0, st>>>(leafflag_t, n, scan_buf); count_launch();
-    scan_exclusive_u32(scan_buf, scan_buf, n, scan_temp, count_dev, st);
-    k_leaf_scatter<<<(n + 255) / 256, 256, 0, st>>>(leafflag_t, scan_buf, n, leaf_start); count_launch();
+    const size_t tn = size_t(T) * n;
+    const unsigned grid = unsigned((tn + 255) / 256);
+    k_flags_u32<<<grid, 256, 0, st>>>(leafflag, tn, scan_buf); count_launch();
+    scan_exclusive_u32(scan_buf, scan_buf, tn, scan_temp, total, st);
+    k_leaf_scatter<<<grid, 256, 0, st>>>(leafflag, scan_buf, tn, n, leaf_start); count_launch();
+    k_leaf_counts<<<(T + 63) / 64, 64, 0, st>>>(scan_buf, total, T, n, counts); count_launch();
 }
 void launch_leaf_pairs(const float* X, int d, int dp, const uint32_t* ids_t,
                        const uint32_t* leaf_start, uint32_t nleaves, uint32_t n, int k,

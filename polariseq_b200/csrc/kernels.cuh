@@ -91,8 +91,8 @@ void launch_leaf_pairs(const float* X, int d, int dp, const uint32_t* ids_t,
                        const uint32_t* leaf_start, uint32_t nleaves, uint32_t n, int k,
                        uint32_t leaf_cap, uint32_t* hidx, float* hdist, uint8_t* hflag,
                        cudaStream_t st);
-void launch_leaf_compact(const uint8_t* leafflag_t, uint32_t n, uint32_t* leaf_start,
-                         uint32_t* scan_buf, void* scan_temp, uint64_t* count_dev,
+void launch_leaf_compact(const uint8_t* leafflag, uint32_t T, uint32_t n, uint32_t* leaf_start,
+                         uint32_t* scan_buf, void* scan_temp, uint64_t* counts, uint64_t* total,
                          cudaStream_t st);
 // Random fill of empty slots (nndescent.rs:820-845).
 void launch_random_fill(const float* X, int d, int dp, uint32_t n, int k, uint64_t seed,
