@@ -59,6 +59,7 @@
 
 #include "ctx.cuh"
 #include "filter.cuh"
+#include "filter_plan.cuh"
 #include "ivf.cuh"
 #include "tc.cuh"
 
@@ -67,12 +68,11 @@ namespace {
 
 constexpr uint32_t FULL = 0xFFFFFFFFu;
 constexpr int FQ = 256;              // queries per job
-constexpr int FC = 128;              // candidates per tile
+constexpr int FC = int(FILTER_TILE); // candidates per tile
 constexpr int FEPI = 512;            // epilogue threads: 2 tile parities x 256 rows
 constexpr int FNT = FEPI + 64;       // + TMA warp + MMA warp
 constexpr int FROWB = 128;           // bytes per operand row and plane (64 BF16)
 constexpr int FMAXCS = 6;            // candidate stages at most
-constexpr int MAX_CHUNKS = 2048;     // chunk maxima per query the bound kernel holds
 constexpr int MAX_SLICES = 16;       // 2 regions per slice: one per lane of a warp
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 
@@ -297,8 +297,6 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
             const uint32_t par = first & 1u;       // all of them have this parity
             float* mrow = PASS == 1 ? a.minima + b.min_off + row : nullptr;
             float run = NEG;
-            // chunks of 128 columns or more: 2^(logc - 7) tiles of one parity
-            const int lt = logc > 7 ? logc - 7 : 0;
             const float ath = PASS == 2 ? a.ath[b.slot + row] : 0.0f;
             const uint32_t cap = S.cap;
             uint32_t* lrow = PASS == 2 ? a.list + b.list_off +
@@ -374,9 +372,8 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
                     }
                 }
                 if constexpr (PASS == 1) {
-                    const uint32_t u = t >> 1;
-                    if (logc >= 7 && (((u + 1) & ((1u << lt) - 1u)) == 0 || t + 2 >= job.t1)) {
-                        mrow[size_t((u >> lt) * 2 + par) * FQ] = run;
+                    if (logc >= 7 && filter_chunk_ends(t, job.t1, uint32_t(logc))) {
+                        mrow[size_t(filter_chunk_slot(t, uint32_t(logc))) * FQ] = run;
                         run = NEG;
                     }
                 }
@@ -861,20 +858,6 @@ cudaError_t launch_bound(uint32_t max_chunks, const FilterSample* s, const FBloc
     return cudaGetLastError();
 }
 
-// Chunk maxima per query: the widest power-of-two chunk (at least 8 columns)
-// that still leaves 4 (k + 1) chunks (the bound then admits about 15 % more
-// than k + 1 points), and at most MAX_CHUNKS.
-uint32_t chunk_count(uint32_t tiles, uint32_t logc) {
-    return logc >= 7 ? 2 * ((tiles + (1u << (logc - 6)) - 1) >> (logc - 6)) : tiles << (7 - logc);
-}
-uint32_t chunk_log(uint32_t n, uint32_t tiles, uint32_t ksel) {
-    const uint64_t want = std::max<uint32_t>(4 * ksel, 64);
-    uint32_t lc = 3;
-    while ((uint64_t(n) >> (lc + 1)) >= want) ++lc;
-    while (chunk_count(tiles, lc) > uint32_t(MAX_CHUNKS)) ++lc;
-    return lc;
-}
-
 // Places per lane of the select kernel's first launch: a quarter more than k + 1.
 int select_places(uint32_t ksel) {
     int kpl = 2;
@@ -914,11 +897,9 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
         FilterSample& s = S[i];
         s.ksel = s.k + 1;
         s.tiles = (s.n + FC - 1) / FC;
-        s.logc = chunk_log(s.n, s.tiles, s.ksel);
-        s.chunks = chunk_count(s.tiles, s.logc);
-        const uint32_t ct = s.logc > 6 ? 1u << (s.logc - 6) : 1u;  // tiles per chunk
-        const uint32_t sl = std::max(1u, std::min(want_slices, s.tiles / 2));
-        slice_tiles[i] = ((s.tiles + sl - 1) / sl + ct - 1) / ct * ct;
+        s.logc = filter_chunk_log(s.n, s.tiles, s.ksel);
+        s.chunks = filter_chunk_count(s.tiles, s.logc);
+        slice_tiles[i] = filter_slice_tiles(s.tiles, s.logc, want_slices);
         s.slices = (s.tiles + slice_tiles[i] - 1) / slice_tiles[i];
         // a region's share of the admitted points is binomial around lambda
         const double lambda = 2.0 * s.ksel / (2.0 * s.slices);
