@@ -4,10 +4,12 @@
 
 #include <stdint.h>
 
+#ifndef PQ_PLAN
 #ifdef __CUDACC__
 #define PQ_PLAN __host__ __device__ __forceinline__
 #else
 #define PQ_PLAN inline
+#endif
 #endif
 
 namespace pq {

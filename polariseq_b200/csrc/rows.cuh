@@ -13,10 +13,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-namespace pq {
+#include "seq_plan.cuh"
 
-// Floats between staged rows of dp floats (dp a multiple of 4).
-__host__ __device__ __forceinline__ int staged_stride(int dp) { return (dp / 4) % 2 ? dp : dp + 4; }
+namespace pq {
 
 // 16-byte asynchronous global -> shared copy (both addresses 16-byte aligned),
 // bypassing L1.

@@ -29,6 +29,7 @@
 #include "common.cuh"
 #include "kernels.cuh"
 #include "rows.cuh"
+#include "seq_plan.cuh"
 
 namespace pq {
 namespace {
@@ -793,15 +794,16 @@ __global__ void __launch_bounds__(NT, NT == BIG_NT ? 2 : 5)
     }
 }
 
+// Static shared memory of a subtree CTA (with room for the compiler's alignment).
+template <int NT, int CAP>
+constexpr size_t SEQ_FIXED = sizeof(SeqShared<NT, CAP>) + 64;
+
 template <int NT, int CAP, int D>
 void seqtree_launch(const ForestArgs& a, const SRoot* roots, uint32_t nr, size_t room,
                     cudaStream_t st) {
     if (nr == 0) return;
-    // as many staged rows (at most CAP) as fit in `room` bytes
-    const size_t row = size_t(staged_stride(a.dp)) * 4;
-    int trows = int(std::min<size_t>(CAP, room / row));
-    if (trows < 2) trows = 0;
-    const size_t dyn = size_t(2 * a.dp) * 4 + row * trows;
+    const int trows = seq_staged_rows(a.dp, CAP, room, SEQ_FIXED<NT, CAP>);
+    const size_t dyn = seq_dynamic(a.dp, trows);
     // (with the static arrays the total passes 48 KB well before dyn does)
     cudaFuncSetAttribute(k_seqtree<NT, CAP, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(dyn));
