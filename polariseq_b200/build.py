@@ -11,6 +11,7 @@ import glob
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -37,15 +38,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     os.makedirs(OUT_DIR, exist_ok=True)
     nvcc = os.environ.get("NVCC", "nvcc")
-    objs = []
-    for src in sources():
+
+    def compile_one(src: str) -> str:
         obj = os.path.join(OUT_DIR, os.path.basename(src)[:-3] + ".o")
         cmd = [nvcc, *ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
                "-ccbin", "g++", "-I", os.path.join(ROOT, "include"), "-c", src, "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         subprocess.run(cmd, check=True)
-        objs.append(obj)
+        return obj
+
+    # the files with the most code first, as many at a time as there are cores
+    srcs = sorted(sources(), key=os.path.getsize, reverse=True)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        objs = sorted(pool.map(compile_one, srcs))
     cmd = [nvcc, *ARCH, "-shared", "-ccbin", "g++", "-o", LIB, *objs, "-lcudart"]
     subprocess.run(cmd, check=True)
     return LIB
