@@ -155,8 +155,10 @@ int pq_ctx_set_profiling(pq_ctx* ctx, int on);
  * with polls > 0, the next tensor-core build's shortlist tile kernels first
  * wait `polls` polls on an mbarrier that nothing arrives at, before issuing
  * any copy or MMA; the wait gives up, the kernels exit with nothing in
- * flight and the build returns PQ_ETIMEOUT.  Applies to one build, after
- * which the context is usable as before. */
+ * flight and the build returns PQ_ETIMEOUT.  An exact or batched search that
+ * uses the tensor-core filter gives up the same way and answers every query
+ * with its full search.  Applies to one call, after which the context is
+ * usable as before. */
 int pq_ctx_set_test_wait(pq_ctx* ctx, uint32_t polls);
 
 /* nndescent_into (nndescent.rs:688-707) with HOST buffers: data is n_obs x

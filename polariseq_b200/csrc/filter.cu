@@ -101,13 +101,14 @@ struct FArgs {
     uint32_t* list;
     uint32_t* cnt;
     int* err;
+    uint32_t test_wait_polls;  // pq_ctx_set_test_wait
 };
 
 struct __align__(8) FBars {
     uint64_t q_full, q_empty;
     uint64_t c_full[FMAXCS], c_empty[FMAXCS];
     uint64_t t_full[2], t_empty[2];
-    uint64_t done;
+    uint64_t done, never;
     uint32_t tmem;
     int abort;
 };
@@ -163,8 +164,11 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
             tc::mbar_init(&B.t_empty[s], FEPI / 64);
         }
         tc::mbar_init(&B.done, 1);
+        tc::mbar_init(&B.never, 1);
         tc::fence_barrier_init();
         B.abort = 0;
+        // the timeout test hook: a bounded wait that runs out before any work
+        if (a.test_wait_polls && !tc::mbar_wait(&B.never, 0, a.test_wait_polls)) B.abort = 1;
     }
     if (tid == FEPI) {
         tc::prefetch_tmap(&tmQ);
@@ -227,7 +231,9 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
             const uint64_t dq = tc::desc_k_sw128(tc::smem_u32(sQ));
             const uint64_t dc0 = tc::desc_k_sw128(tc::smem_u32(sC));
             uint32_t qi = 0, ci = 0, ti = 0;
-            for (uint32_t j = blockIdx.x; j < a.njobs && !*abort_flag; j += gridDim.x) {
+            for (uint32_t j = blockIdx.x; j < a.njobs; j += gridDim.x) {
+                // (one decision per warp: its lanes may read the flag apart)
+                if (__any_sync(FULL, *abort_flag)) break;
                 const uint32_t t0 = a.jobs[j].t0, t1 = a.jobs[j].t1;
                 bool ok = __all_sync(FULL, tc::mbar_wait(&B.q_full, qi & 1, WAIT_LIMIT));
                 for (uint32_t t = t0; t < t1 && ok; ++t) {
@@ -287,7 +293,8 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
             taddr + (uint32_t((w & 3) * 32) << 16) + uint32_t(grp * 2 * FC + h * FC);
         const float NEG = __int_as_float(0xff800000);
         uint32_t ti = 0;  // tiles of the CTA before this job
-        for (uint32_t j = blockIdx.x; j < a.njobs && !*abort_flag; j += gridDim.x) {
+        for (uint32_t j = blockIdx.x; j < a.njobs; j += gridDim.x) {
+            if (__any_sync(FULL, *abort_flag)) break;
             const FJob job = a.jobs[j];
             const FBlock b = a.blocks[job.block];
             const FilterSample& S = a.samples[b.sample];
@@ -1062,6 +1069,8 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     fa.list = list;
     fa.cnt = cnt;
     fa.err = flags + ns;
+    fa.test_wait_polls = c->test_wait_polls;
+    c->test_wait_polls = 0;  // the hook applies to one call
     SelArgs sa{};
     sa.samples = ds;
     sa.list = list;

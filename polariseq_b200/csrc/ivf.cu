@@ -327,7 +327,9 @@ __global__ void __launch_bounds__(NT, 1) k_ivf_tiles(const __grid_constant__ CUt
             }
         };
         load_job(blockIdx.x);
-        for (uint32_t job = blockIdx.x; job < a.njobs && !*abort_flag; job += gridDim.x) {
+        for (uint32_t job = blockIdx.x; job < a.njobs; job += gridDim.x) {
+            // (one decision per warp: its lanes may read the flag apart)
+            if (__any_sync(FULL, *abort_flag)) break;
             const uint32_t b = nb, qs = nqs, qe = nqe, ts = nts;
             load_job(job + gridDim.x);
             const uint32_t cs = a.c_off[b], ce = a.c_off[b + 1];
@@ -768,7 +770,9 @@ __global__ void __launch_bounds__(WNT, 1) k_ivf_wide(const __grid_constant__ CUt
             }
         };
         load_job(blockIdx.x);
-        for (uint32_t job = blockIdx.x; job < a.njobs && !*abort_flag; job += gridDim.x) {
+        for (uint32_t job = blockIdx.x; job < a.njobs; job += gridDim.x) {
+            // (one decision per warp: its lanes may read the flag apart)
+            if (__any_sync(FULL, *abort_flag)) break;
             const uint32_t b = nb, qs = nqs, qe = nqe, ts = nts;
             load_job(job + gridDim.x);
             const uint32_t cs = a.c_off[b], ce = a.c_off[b + 1];
