@@ -792,7 +792,8 @@ bool prepare_exact_filter(pq_ctx* c, const float* X, uint64_t n, uint64_t d, uin
         out->redo_ld = uint32_t(ld);
         out->redo_cap = uint32_t(std::max<uint64_t>(
             64, std::min<uint64_t>((n + 7) / 8, (uint64_t(1) << 30) / (ld * 4)) / 4 * 4));
-        out->redo_dist = c->get<float>("ex_redo_d", out->redo_cap * ld);
+        out->redo_dist = c->get<float>(
+            "ex_redo_d", std::max<uint64_t>(out->redo_cap * ld, pq::exact_redo_floats(uint32_t(ld))));
         return true;
     } catch (const std::string&) {
         return false;

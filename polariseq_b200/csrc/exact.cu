@@ -230,10 +230,10 @@ __global__ void __launch_bounds__(EW * 32) k_exact_knn(const float* __restrict__
 // barriers (346 us for 17 queries at 20,000 x 50, 4.6 ms for 2,762 at 60,013 x
 // 30 cosine).  The distance buffer holds redo_cap queries; k_redo_rest takes
 // those past them.
-constexpr int RQ = 4;     // queries per CTA of k_redo_dist
-constexpr int RD = 256;   // candidates (= threads) per CTA
+constexpr int RQ = int(EXACT_REDO_Q);  // queries per CTA of k_redo_dist
+constexpr int RD = 256;                // candidates (= threads) per CTA
 
-// dist[u * ld + j] of RQ queries (their rows in sq, dimension-major) and row j;
+// dist[u * ld] of RQ queries (their rows in sq, dimension-major) and row j;
 // rows are column-major, so every load is one coalesced line.
 template <int D>
 __device__ __forceinline__ void redo_dist4(const float* __restrict__ Xt, uint32_t n, int d_,
@@ -283,7 +283,7 @@ __device__ __forceinline__ void redo_dist4(const float* __restrict__ Xt, uint32_
             const float den = __fmul_rn(__fsqrt_rn(qn[u]), __fsqrt_rn(norms[j]));
             r = den > 0.0f ? __fsub_rn(1.0f, __fdiv_rn(r, den)) : 1.0f;
         }
-        dist[size_t(u) * ld + j] = r;
+        dist[size_t(u) * ld] = r;
     }
 }
 
@@ -299,14 +299,11 @@ __device__ __forceinline__ void redo_queries(const float* __restrict__ Xt, uint3
         qn[threadIdx.x] = cosine ? norms[list[min(i0 + threadIdx.x, nq - 1)]] : 0.0f;
 }
 
-// One warp: the sequential scan over a query's distances (512 in flight, 128
-// per vote), then its output row.
-__device__ __forceinline__ void redo_replay(const float* __restrict__ row, uint32_t n, int kws,
-                                            int cosine, uint32_t q, float* hd, uint32_t* hi,
-                                            uint32_t* __restrict__ out_idx,
-                                            float* __restrict__ out_dist) {
+// One warp: the sequential scan over a query's distances to candidates [c0, c0 +
+// n) (512 in flight, 128 per vote).
+__device__ __forceinline__ void redo_scan(const float* __restrict__ row, uint32_t c0, uint32_t n,
+                                          int kws, float* hd, uint32_t* hi, int& hlen) {
     const int lane = threadIdx.x & 31;
-    int hlen = 0;
     for (uint32_t j0 = 0; j0 < n; j0 += 512) {
         float dd[16];
 #pragma unroll
@@ -324,12 +321,10 @@ __device__ __forceinline__ void redo_replay(const float* __restrict__ row, uint3
             for (int g = 4 * v; g < 4 * v + 4; ++g) {
                 const uint32_t jg = j0 + 32 * g;
                 if (jg < n)
-                    replay_tile(hd, hi, hlen, kws, dd[g], jg, n - jg < 32 ? n - jg : 32, lane);
+                    replay_tile(hd, hi, hlen, kws, dd[g], c0 + jg, n - jg < 32 ? n - jg : 32, lane);
             }
         }
     }
-    write_row(hd, hi, hlen, kws, q, cosine, lane, out_idx, out_dist);
-    __syncwarp();
 }
 
 // The first cap queries of the list: distances over the whole grid ...
@@ -348,7 +343,7 @@ __global__ void __launch_bounds__(RD) k_redo_dist(const float* __restrict__ Xt, 
         redo_queries(Xt, n, d, cosine, norms, list, nq, i0, sq, qn);
         __syncthreads();
         if (j < n)
-            redo_dist4<D>(Xt, n, d, cosine, norms, sq, qn, j, ld, dist + size_t(i0) * ld);
+            redo_dist4<D>(Xt, n, d, cosine, norms, sq, qn, j, ld, dist + size_t(i0) * ld + j);
     }
 }
 // ... and their scans, a warp each.
@@ -361,18 +356,25 @@ __global__ void __launch_bounds__(32) k_redo_replay(const float* __restrict__ di
     __shared__ float hd[EXACT_MAX_K];
     __shared__ uint32_t hi[EXACT_MAX_K];
     const uint32_t nq = min(*list_n, cap);
-    for (uint32_t i = blockIdx.x; i < nq; i += gridDim.x)
-        redo_replay(dist + size_t(i) * ld, n, kws, cosine, list[i], hd, hi, out_idx, out_dist);
+    for (uint32_t i = blockIdx.x; i < nq; i += gridDim.x) {
+        int hlen = 0;
+        redo_scan(dist + size_t(i) * ld, 0, n, kws, hd, hi, hlen);
+        write_row(hd, hi, hlen, kws, list[i], cosine, threadIdx.x, out_idx, out_dist);
+        __syncwarp();
+    }
 }
-// The queries past the first cap (inputs full of ties): RQ per CTA at a time,
-// their distances in the CTA's own rows of the buffer.
+// The queries past the first cap (inputs full of ties, or that the filter's
+// bounds do not cover): RQ per CTA at a time, EXACT_REDO_SEG candidates after
+// another through the CTA's own part of the buffer, so that the grid fills the
+// chip whatever the number of points.  (With whole rows per CTA the buffer held
+// 134 CTAs at 500,000 points.)
 template <int D>
 __global__ void __launch_bounds__(RD) k_redo_rest(const float* __restrict__ Xt, uint32_t n, int d,
                                                   int kws, int cosine,
                                                   const float* __restrict__ norms,
                                                   const uint32_t* __restrict__ list,
                                                   const uint32_t* __restrict__ list_n,
-                                                  uint32_t cap, uint32_t ld,
+                                                  uint32_t cap, uint32_t seg,
                                                   float* __restrict__ dist,
                                                   uint32_t* __restrict__ out_idx,
                                                   float* __restrict__ out_dist) {
@@ -381,17 +383,23 @@ __global__ void __launch_bounds__(RD) k_redo_rest(const float* __restrict__ Xt, 
     __shared__ float hd[RQ][EXACT_MAX_K];
     __shared__ uint32_t hi[RQ][EXACT_MAX_K];
     const uint32_t nq = *list_n, w = threadIdx.x >> 5;
-    float* mine = dist + size_t(blockIdx.x) * RQ * ld;
+    float* mine = dist + size_t(blockIdx.x) * RQ * seg;
     for (uint32_t i0 = cap + blockIdx.x * RQ; i0 < nq; i0 += gridDim.x * RQ) {
         __syncthreads();
         redo_queries(Xt, n, d, cosine, norms, list, nq, i0, sq, qn);
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < n; j += RD)
-            redo_dist4<D>(Xt, n, d, cosine, norms, sq, qn, j, ld, mine);
-        __syncthreads();
-        if (w < uint32_t(RQ) && i0 + w < nq)
-            redo_replay(mine + size_t(w) * ld, n, kws, cosine, list[i0 + w], hd[w], hi[w], out_idx,
-                        out_dist);
+        const bool scans = w < uint32_t(RQ) && i0 + w < nq;
+        int hlen = 0;
+        for (uint32_t c0 = 0; c0 < n; c0 += seg) {
+            const uint32_t len = min(seg, n - c0);
+            __syncthreads();  // the queries are there, the last segment is scanned
+            for (uint32_t j = threadIdx.x; j < len; j += RD)
+                redo_dist4<D>(Xt, n, d, cosine, norms, sq, qn, c0 + j, seg, mine + j);
+            __syncthreads();
+            if (scans) redo_scan(mine + size_t(w) * seg, c0, len, kws, hd[w], hi[w], hlen);
+        }
+        if (scans)
+            write_row(hd[w], hi[w], hlen, kws, list[i0 + w], cosine, threadIdx.x & 31, out_idx,
+                      out_dist);
     }
 }
 
@@ -419,9 +427,9 @@ cudaError_t launch_d(const float* X, uint64_t n, int d, int kws, int cosine, flo
                                             filter->redo_n, cap, ld, filter->redo_dist);
         k_redo_replay<<<148 * 16, 32, 0, st>>>(filter->redo_dist, uint32_t(n), ld, kws, cosine,
                                               filter->redo, filter->redo_n, cap, indices, dists);
-        k_redo_rest<D><<<std::min<uint32_t>(cap / RQ, 148 * 4), RD, 0, st>>>(
-            filter->Xt, uint32_t(n), d, kws, cosine, norms, filter->redo, filter->redo_n, cap, ld,
-            filter->redo_dist, indices, dists);
+        k_redo_rest<D><<<EXACT_REDO_CTAS, RD, 0, st>>>(
+            filter->Xt, uint32_t(n), d, kws, cosine, norms, filter->redo, filter->redo_n, cap,
+            std::min(EXACT_REDO_SEG, ld), filter->redo_dist, indices, dists);
         count_launch();
         count_launch();
         count_launch();

@@ -26,9 +26,16 @@ struct ExactFilter {
     uint32_t* redo;    // device: query rows
     uint32_t* redo_n;  // device: their number
     const float* Xt;   // device: the rows column-major [d][n], written by `run`
-    float* redo_dist;  // device: distances of redo_cap queries, redo_ld apart
+    float* redo_dist;  // device: distances of redo_cap queries, redo_ld apart; at least
+                       // exact_redo_floats(redo_ld) floats for the queries past them
     uint32_t redo_cap, redo_ld;
 };
+constexpr uint32_t EXACT_REDO_Q = 4;          // queries at a time per CTA
+constexpr uint32_t EXACT_REDO_SEG = 8192;     // their candidates at a time
+constexpr uint32_t EXACT_REDO_CTAS = 148 * 4;
+inline size_t exact_redo_floats(uint32_t ld) {
+    return size_t(EXACT_REDO_CTAS) * EXACT_REDO_Q * (ld < EXACT_REDO_SEG ? ld : EXACT_REDO_SEG);
+}
 cudaError_t launch_exact_knn(const float* X, uint64_t n, int d, int kws, int cosine,
                              float* norms, uint32_t* indptr, uint32_t* indices, float* dists,
                              cudaStream_t st, const ExactFilter* filter = nullptr);
