@@ -781,8 +781,8 @@ bool prepare_exact_filter(pq_ctx* c, const float* X, uint64_t n, uint64_t d, uin
         f.samples.push_back(s);
         f.out_idx = indices;
         f.out_dist = dists;
-        out->redo = f.redo_a = c->get<uint32_t>("ex_redo", n);
-        out->redo_n = f.redo_count = c->get<uint32_t>("ex_redo_n", 1);
+        out->redo = f.redo_rows = c->get<uint32_t>("ex_redo", n);
+        out->redo_n = f.redo_rows_n = c->get<uint32_t>("ex_redo_n", 1);
         pq::FilterPlan plan = pq::filter_prepare(c, std::move(f));
         out->run = plan.run;
         out->Xt = plan.Xt;
@@ -1172,9 +1172,11 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
         if (it != c->batch_shape.end() && !(flags & PQ_BATCH_AUTOTUNE)) {
             shape = it->second;
         } else if (n_taken == n_samples && !(flags & PQ_BATCH_AUTOTUNE)) {
-            // only left-over blocks would use the shape: not worth timing
-            for (int sh = pq::batched_shapes() - 1; sh >= 0 && shape < 0; --sh)
-                if (pq::batched_shape_fits(sh, int(d), kp)) shape = sh;
+            // only left-over blocks would use the shape: not worth timing.  What the
+            // timing chooses most (600 to 240,000 points, k 10 to 400): 8 warps of 4
+            // queries, of 8 queries at k 32 to 128 with enough blocks for the chip.
+            shape = kp > 32 && kp <= 128 && offsets[n_samples] >= 20000 ? 3 : 2;
+            while (shape >= 0 && !pq::batched_shape_fits(shape, int(d), kp)) --shape;
             if (shape < 0) throw DeviceError{"no tile shape fits this k and n_dim"};
         } else {
             float best = 0.f;
@@ -1211,14 +1213,30 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
         std::function<cudaError_t(cudaStream_t)> filter;
         if (n_taken > 0) {
             try {
+                // the full search's items: those of the samples it takes whole, then
+                // those of the filter's samples, searched where the filter says so
                 items_for(shape, is, iq);
-                const size_t all_items = is.size();
-                uint32_t* redo_s = c->get<uint32_t>("bt_redo_s", all_items);
-                uint32_t* redo_q = c->get<uint32_t>("bt_redo_q", all_items);
-                uint32_t* redo_n = c->get<uint32_t>("bt_redo_n", 2);  // blocks, single queries
+                const uint32_t qpi = uint32_t(pq::batched_queries_per_item(shape));
+                std::vector<uint32_t> fs, fq;
+                std::vector<uint64_t> off(n_samples, 0);
+                size_t o = 0;
+                for (size_t i = 0; i < is.size(); ++i) {
+                    if (taken[is[i]]) {
+                        if (iq[i] == 0) off[is[i]] = fs.size();
+                        fs.push_back(is[i]);
+                        fq.push_back(iq[i]);
+                    } else {
+                        is[o] = is[i];
+                        iq[o++] = iq[i];
+                    }
+                }
+                is.resize(o);
+                iq.resize(o);
+                is.insert(is.end(), fs.begin(), fs.end());
+                iq.insert(iq.end(), fq.begin(), fq.end());
+                upload_items(uint32_t(is.size()));
                 // (a group whose rows the filter cannot bound has more queries)
                 const uint32_t few = 512;
-                uint2* redo_1 = c->get<uint2>("bt_redo_1", few);
                 pq::FilterCall f{};
                 f.X = d_data;
                 f.rows = offsets[n_samples];
@@ -1233,48 +1251,25 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
                     g.k = ks[s];
                     f.samples.push_back(g);
                     f.ids.push_back(s);
+                    f.redo_off.push_back(off[s]);
                 }
                 f.out_idx = d_indices;
                 f.out_dist = d_dists;
-                f.redo_block = uint32_t(pq::batched_queries_per_item(shape));
-                f.redo_a = redo_s;
-                f.redo_b = redo_q;
-                f.redo_count = redo_n;
-                f.redo_queries = redo_1;
-                f.redo_queries_n = redo_n + 1;
+                f.redo_block = qpi;
+                f.redo_flag = c->get<uint32_t>("bt_redo_flag", fs.size());
+                f.redo_flags = fs.size();
+                f.redo_queries = c->get<uint2>("bt_redo_1", few);
+                f.redo_queries_n = c->get<uint32_t>("bt_redo_n", 1);
                 f.redo_short = few;
-                filter = pq::filter_prepare(c, std::move(f)).run;
-                // the full search's items of the samples it takes whole, at the
-                // head of the list; the filter appends to them
-                size_t o = 0;
-                for (size_t i = 0; i < is.size(); ++i)
-                    if (!taken[is[i]]) {
-                        is[o] = is[i];
-                        iq[o++] = iq[i];
-                    }
-                is.resize(o);
-                iq.resize(o);
-                uint32_t* first = c->get<uint32_t>("bt_first_n", 2);
-                const uint32_t o32[2] = {uint32_t(o), 0u};
-                ck(cudaMemcpyAsync(first, o32, 8, cudaMemcpyHostToDevice, st), "h2d");
-                ck(cudaMemcpyAsync(redo_s, is.data(), o * 4, cudaMemcpyHostToDevice, st), "h2d");
-                ck(cudaMemcpyAsync(redo_q, iq.data(), o * 4, cudaMemcpyHostToDevice, st), "h2d");
-                b.item_s = redo_s;
-                b.item_q = redo_q;
-                b.n_items = uint32_t(all_items);
-                b.items_dev = redo_n;
-                b.first_dev = first;
-                b.single = redo_1;
-                b.single_n = redo_n + 1;
+                b.first = uint32_t(o);
+                b.single = f.redo_queries;
+                b.single_n = f.redo_queries_n;
                 b.single_max = few;
-                auto run = filter;
-                filter = [=](cudaStream_t q) {
-                    cudaError_t e = cudaMemcpyAsync(redo_n, first, 8, cudaMemcpyDeviceToDevice, q);
-                    return e == cudaSuccess ? run(q) : e;
-                };
+                const uint32_t* flag = f.redo_flag;
+                filter = pq::filter_prepare(c, std::move(f)).run;
+                b.flag = flag;
             } catch (const std::string&) {  // no room for the filter's workspace
                 filter = nullptr;
-                b.items_dev = nullptr;
             }
         }
         if (!filter) {

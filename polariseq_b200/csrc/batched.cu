@@ -25,7 +25,8 @@
 //
 // This full search takes the samples the tensor-core filter (filter.cu) does
 // not: d > 62 or fewer than 16 points per neighbour; and the query blocks that
-// the filter leaves, whose number only the device knows (items_dev).
+// the filter leaves, which only the device knows (a flag per block: the blocks
+// keep their order, sample after sample, in which CTAs share candidates in L2).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -51,10 +52,10 @@ struct BatchArgs {
     const uint32_t* item_s;  // work item: sample
     const uint32_t* item_q;  // work item: first local query
     uint32_t n_items;
-    // optional: the number of items, on the device; items past the first
-    // *first_dev only when *single_n queries are too many for k_batched_redo
-    const uint32_t* items_dev;
-    const uint32_t* first_dev;
+    // optional: items past the first `first` are searched where their flag is
+    // set, and only when *single_n queries are too many for k_batched_redo
+    const uint32_t* flag;
+    uint32_t first;
     const uint2* single;
     const uint32_t* single_n;
     uint32_t single_max;
@@ -152,14 +153,14 @@ __global__ void __launch_bounds__(NW * 32) k_batched_knn(BatchArgs a) {
     __shared__ uint32_t s_item;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kp = a.kp;
-    const uint32_t n_items = !a.items_dev ? a.n_items
-                             : *a.single_n < a.single_max ? *a.first_dev : *a.items_dev;
+    const uint32_t n_items = a.flag && *a.single_n < a.single_max ? a.first : a.n_items;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1u);
         __syncthreads();
         const uint32_t item = s_item;
         __syncthreads();
         if (item >= n_items) break;
+        if (a.flag && item >= a.first && !a.flag[item - a.first]) continue;
         const uint32_t s = a.item_s[item], q0 = a.item_q[item];
         const uint64_t base = a.s_off[s];
         const uint32_t ns = uint32_t(a.s_off[s + 1] - base);
@@ -481,8 +482,8 @@ cudaError_t launch_batched_knn(const BatchLaunch& b, int shape, cudaStream_t st)
     a.item_s = b.item_s;
     a.item_q = b.item_q;
     a.n_items = b.n_items;
-    a.items_dev = b.items_dev;
-    a.first_dev = b.first_dev;
+    a.flag = b.flag;
+    a.first = b.first;
     a.single = b.single;
     a.single_n = b.single_n;
     a.single_max = b.single_max;
@@ -490,7 +491,7 @@ cudaError_t launch_batched_knn(const BatchLaunch& b, int shape, cudaStream_t st)
     a.kp = b.kp;
     a.out_idx = b.out_idx;
     a.out_dist = b.out_dist;
-    if (b.items_dev) {
+    if (b.flag) {
         k_batched_redo<<<std::min<uint32_t>(b.single_max, uint32_t(b.sms) * 2), RW + 32,
                          size_t(b.kp) * 8, st>>>(a);
         count_launch();

@@ -16,12 +16,11 @@ struct BatchLaunch {
     const uint32_t* item_s;  // device: work item -> sample
     const uint32_t* item_q;  // device: work item -> first local query
     uint32_t n_items;
-    // optional, device: the number of items (at most n_items), how many of them
-    // come first whatever else happens, and single queries (sample, query) that
-    // are searched one by one instead of the other items when there are fewer
-    // than single_max
-    const uint32_t* items_dev;
-    const uint32_t* first_dev;
+    // optional, device: a flag per item past the first `first` (the others are
+    // left out), and the single queries (sample, query) that the flags stand for:
+    // fewer than single_max are searched one by one instead
+    const uint32_t* flag;
+    uint32_t first;
     const uint2* single;
     const uint32_t* single_n;
     uint32_t single_max;

@@ -364,10 +364,10 @@ __global__ void __launch_bounds__(32) k_redo_replay(const float* __restrict__ di
     }
 }
 // The queries past the first cap (inputs full of ties, or that the filter's
-// bounds do not cover): RQ per CTA at a time, EXACT_REDO_SEG candidates after
-// another through the CTA's own part of the buffer, so that the grid fills the
-// chip whatever the number of points.  (With whole rows per CTA the buffer held
-// 134 CTAs at 500,000 points.)
+// bounds do not cover): RQ per CTA at a time, `seg` candidates after another
+// through the CTA's own part of the buffer, so that the grid fills the chip
+// whatever the number of points.  (With whole rows per CTA the buffer held 134
+// CTAs at 500,000 points.)
 template <int D>
 __global__ void __launch_bounds__(RD) k_redo_rest(const float* __restrict__ Xt, uint32_t n, int d,
                                                   int kws, int cosine,
@@ -429,7 +429,7 @@ cudaError_t launch_d(const float* X, uint64_t n, int d, int kws, int cosine, flo
                                               filter->redo, filter->redo_n, cap, indices, dists);
         k_redo_rest<D><<<EXACT_REDO_CTAS, RD, 0, st>>>(
             filter->Xt, uint32_t(n), d, kws, cosine, norms, filter->redo, filter->redo_n, cap,
-            std::min(EXACT_REDO_SEG, ld), filter->redo_dist, indices, dists);
+            exact_redo_seg(ld), filter->redo_dist, indices, dists);
         count_launch();
         count_launch();
         count_launch();

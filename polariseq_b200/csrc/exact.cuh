@@ -31,10 +31,14 @@ struct ExactFilter {
     uint32_t redo_cap, redo_ld;
 };
 constexpr uint32_t EXACT_REDO_Q = 4;          // queries at a time per CTA
-constexpr uint32_t EXACT_REDO_SEG = 8192;     // their candidates at a time
 constexpr uint32_t EXACT_REDO_CTAS = 148 * 4;
+// Their candidates at a time: whole rows while those of every CTA fit in 620 MB,
+// else 8,192.  (Segments of 8,192 at 60,000 points: 48.6 -> 44.8 ms with a zero
+// row at k = 15, but 19.6 -> 20.1 with ties at k = 100, where the scans' barriers
+// count; at 200,000 points 727 -> 475.)
+inline uint32_t exact_redo_seg(uint32_t ld) { return ld <= 65536 ? ld : 8192; }
 inline size_t exact_redo_floats(uint32_t ld) {
-    return size_t(EXACT_REDO_CTAS) * EXACT_REDO_Q * (ld < EXACT_REDO_SEG ? ld : EXACT_REDO_SEG);
+    return size_t(EXACT_REDO_CTAS) * EXACT_REDO_Q * exact_redo_seg(ld);
 }
 cudaError_t launch_exact_knn(const float* X, uint64_t n, int d, int kws, int cosine,
                              float* norms, uint32_t* indptr, uint32_t* indices, float* dists,

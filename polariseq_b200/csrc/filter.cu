@@ -88,6 +88,7 @@ struct FBlock {       // 256 queries of one group
 
 struct FJob {
     uint32_t block, slice, t0, t1;  // tiles [t0, t1)
+    uint32_t sample, pad;
 };
 
 struct FArgs {
@@ -95,6 +96,7 @@ struct FArgs {
     const FBlock* blocks;
     const FJob* jobs;
     uint32_t njobs;
+    const int* odd;     // groups that go to the full search whole: their jobs are left out
     uint32_t plane;     // rows between the hi and lo planes (two-plane operands)
     float* minima;
     const float* ath;   // per query slot: the admission bound
@@ -184,8 +186,10 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
             uint32_t qi = 0, ci = 0;
             for (uint32_t j = blockIdx.x; j < a.njobs && !*abort_flag; j += gridDim.x) {
                 const FJob job = a.jobs[j];
+                const int odd = a.odd[job.sample];  // (read beside the block)
                 const FBlock b = a.blocks[job.block];
-                const uint32_t base = uint32_t(a.samples[b.sample].base);
+                const uint32_t base = uint32_t(a.samples[job.sample].base);
+                if (odd) continue;
                 if (!tc::mbar_wait(&B.q_empty, (qi & 1) ^ 1, WAIT_LIMIT)) {
                     *abort_flag = 1;
                     break;
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
             for (uint32_t j = blockIdx.x; j < a.njobs; j += gridDim.x) {
                 // (one decision per warp: its lanes may read the flag apart)
                 if (__any_sync(FULL, *abort_flag)) break;
+                if (a.odd[a.jobs[j].sample]) continue;
                 const uint32_t t0 = a.jobs[j].t0, t1 = a.jobs[j].t1;
                 bool ok = __all_sync(FULL, tc::mbar_wait(&B.q_full, qi & 1, WAIT_LIMIT));
                 for (uint32_t t = t0; t < t1 && ok; ++t) {
@@ -296,9 +301,11 @@ __global__ void __launch_bounds__(FNT, 1) k_filter_tiles(const __grid_constant__
         for (uint32_t j = blockIdx.x; j < a.njobs; j += gridDim.x) {
             if (__any_sync(FULL, *abort_flag)) break;
             const FJob job = a.jobs[j];
+            const int odd = a.odd[job.sample];
             const FBlock b = a.blocks[job.block];
-            const FilterSample& S = a.samples[b.sample];
+            const FilterSample& S = a.samples[job.sample];
             const int n = int(S.n), logc = int(S.logc);
+            if (odd) continue;
             const uint32_t skip = (ti ^ uint32_t(grp)) & 1u;
             const uint32_t first = job.t0 + skip;  // this group's first tile
             const uint32_t par = first & 1u;       // all of them have this parity
@@ -508,8 +515,10 @@ __global__ void __launch_bounds__(256) k_filter_bound(const FilterSample* __rest
                                                       const FBlock* __restrict__ blocks,
                                                       const float* __restrict__ minima,
                                                       const float* __restrict__ qn, float abs_m,
+                                                      const int* __restrict__ odd,
                                                       float* __restrict__ ath) {
     const FBlock b = blocks[blockIdx.x >> 5];
+    if (odd[b.sample]) return;
     const FilterSample& S = samples[b.sample];
     const int lane = threadIdx.x & 31;
     const uint32_t row = (blockIdx.x & 31) * 8 + (threadIdx.x >> 5), q = b.q0 + row;
@@ -625,16 +634,16 @@ struct SelArgs {
     const int* err;
     uint32_t* out_idx;
     float* out_dist;
+    // FilterCall's, for the queries that go to the full search
     const uint32_t* ids;
+    const uint64_t* redo_off;
     uint32_t redo_block;
-    uint32_t* redo_a;
-    uint32_t* redo_b;
-    uint32_t* redo_count;
-    uint2* redo_queries;        // FILTER_BATCHED: (group id, query), the first redo_short
+    uint32_t* redo_flag;
+    uint2* redo_queries;
     uint32_t* redo_queries_n;
     uint32_t redo_short;
-    uint32_t* redo_flag;        // FILTER_BATCHED: one per redo block of a group
-    const uint64_t* redo_off;   // FILTER_BATCHED: first flag of each group
+    uint32_t* redo_rows;
+    uint32_t* redo_rows_n;
     uint32_t block0;            // first block of the launch
     // lists too long for the first launch's places: (block, row) pairs for a
     // second launch with four times the places
@@ -797,16 +806,14 @@ __device__ __forceinline__ void select_query(const SelArgs& a, uint32_t block, u
     }
     if (bad && lane == 0) {
         if constexpr (MODE == FILTER_BATCHED) {
-            const uint32_t blk = q / a.redo_block;
-            if (atomicExch(&a.redo_flag[a.redo_off[b.sample] + blk], 1u) == 0u) {
-                const uint32_t i = atomicAdd(a.redo_count, 1u);
-                a.redo_a[i] = a.ids[b.sample];
-                a.redo_b[i] = blk * a.redo_block;
+            a.redo_flag[a.redo_off[b.sample] + q / a.redo_block] = 1u;
+            // (once there are too many, their number no longer matters)
+            if (*static_cast<volatile uint32_t*>(a.redo_queries_n) < a.redo_short) {
+                const uint32_t i = atomicAdd(a.redo_queries_n, 1u);
+                if (i < a.redo_short) a.redo_queries[i] = make_uint2(a.ids[b.sample], q);
             }
-            const uint32_t i = atomicAdd(a.redo_queries_n, 1u);
-            if (i < a.redo_short) a.redo_queries[i] = make_uint2(a.ids[b.sample], q);
         } else {
-            a.redo_a[atomicAdd(a.redo_count, 1u)] = q;
+            a.redo_rows[atomicAdd(a.redo_rows_n, 1u)] = q;
         }
     }
 }
@@ -899,12 +906,16 @@ cudaError_t launch_tiles(int ks, const CUtensorMap& q, const CUtensorMap& c, con
 
 cudaError_t launch_bound(uint32_t max_chunks, const FilterSample* s, const FBlock* b,
                          uint32_t blocks, const float* minima, const float* qn, float abs_m,
-                         float* ath, cudaStream_t st) {
+                         const int* odd, float* ath, cudaStream_t st) {
     const unsigned g = blocks * 32;
-    if (max_chunks <= 128) k_filter_bound<4><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, ath);
-    else if (max_chunks <= 512) k_filter_bound<16><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, ath);
-    else if (max_chunks <= 1024) k_filter_bound<32><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, ath);
-    else k_filter_bound<64><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, ath);
+    if (max_chunks <= 128)
+        k_filter_bound<4><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, odd, ath);
+    else if (max_chunks <= 512)
+        k_filter_bound<16><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, odd, ath);
+    else if (max_chunks <= 1024)
+        k_filter_bound<32><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, odd, ath);
+    else
+        k_filter_bound<64><<<g, 256, 0, st>>>(s, b, minima, qn, abs_m, odd, ath);
     count_launch();
     return cudaGetLastError();
 }
@@ -941,8 +952,7 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     const uint32_t want_slices =
         uint32_t(std::min<uint64_t>(MAX_SLICES, (4 * uint64_t(sms) + qblocks - 1) / qblocks));
     uint32_t max_chunks = 0;
-    uint64_t nflags = 0;
-    std::vector<uint64_t> redo_off(ns);
+    const uint64_t nflags = call.mode == FILTER_BATCHED ? call.redo_flags : 0;
     std::vector<uint32_t> slice_tiles(ns);
     for (uint32_t i = 0; i < ns; ++i) {
         FilterSample& s = S[i];
@@ -970,8 +980,6 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
         }
         s.inv = uint32_t(x0 < 0 ? x0 + int64_t(s.n) : x0);
         max_chunks = std::max(max_chunks, s.chunks);
-        redo_off[i] = nflags;
-        if (call.mode == FILTER_BATCHED) nflags += (s.n + call.redo_block - 1) / call.redo_block;
     }
     // groups largest first, then their query blocks, in rounds whose chunk
     // maxima and lists stay within 1.5 GB of workspace (at least one block each)
@@ -1012,7 +1020,7 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
                 kpl.push_back(uint8_t(select_places(s.ksel)));
                 for (uint32_t x = 0; x < s.slices; ++x)
                     jobs.push_back(FJob{local, x, x * slice_tiles[i],
-                                        std::min(s.tiles, (x + 1) * slice_tiles[i])});
+                                        std::min(s.tiles, (x + 1) * slice_tiles[i]), i, 0});
                 um += m;
                 ul += l;
                 uc += cn;
@@ -1034,7 +1042,7 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     FilterSample* ds = up("ft_samples", S);
     FBlock* dbk = up("ft_blocks", blocks);
     FJob* dj = up("ft_jobs", jobs);
-    uint64_t* dro = up("ft_redo_off", redo_off);
+    uint64_t* dro = up("ft_redo_off", call.redo_off);
     uint32_t* dids = up("ft_ids", call.ids);
     const uint64_t oprow = uint64_t(kb) * rows;
     __nv_bfloat16* Q = c->get<__nv_bfloat16>("ft_q", oprow * 64);
@@ -1044,7 +1052,6 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     float* qn = c->get<float>("ft_qn", rows);
     float* mean = c->get<float>("ft_mean", size_t(ns) * 64);
     int* flags = c->get<int>("ft_flags", size_t(ns) + 1);  // odd groups, then the abort flag
-    uint32_t* redo_flag = c->get<uint32_t>("ft_redo_flag", std::max<uint64_t>(nflags, 1));
     float* minima = c->get<float>("ft_min", max_min);
     uint32_t* list = c->get<uint32_t>("ft_list", max_list);
     uint32_t* cnt = c->get<uint32_t>("ft_cnt", max_cnt);
@@ -1068,6 +1075,7 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     fa.ath = ath;
     fa.list = list;
     fa.cnt = cnt;
+    fa.odd = flags;
     fa.err = flags + ns;
     fa.test_wait_polls = c->test_wait_polls;
     c->test_wait_polls = 0;  // the hook applies to one call
@@ -1085,15 +1093,14 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     sa.out_idx = call.out_idx;
     sa.out_dist = call.out_dist;
     sa.ids = dids;
+    sa.redo_off = dro;
     sa.redo_block = call.redo_block;
-    sa.redo_a = call.redo_a;
-    sa.redo_b = call.redo_b;
-    sa.redo_count = call.redo_count;
+    sa.redo_flag = call.redo_flag;
     sa.redo_queries = call.redo_queries;
     sa.redo_queries_n = call.redo_queries_n;
     sa.redo_short = call.redo_short;
-    sa.redo_flag = redo_flag;
-    sa.redo_off = dro;
+    sa.redo_rows = call.redo_rows;
+    sa.redo_rows_n = call.redo_rows_n;
     sa.longer = c->get<uint32_t>("ft_longer", max_slots);
     sa.longer_n = c->get<uint32_t>("ft_longer_n", 1);
     // the FP32 distance errs by a part of the distance (Euclidean) or by at
@@ -1103,7 +1110,9 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     auto run = [=](cudaStream_t s) -> cudaError_t {
         cudaError_t e;
         if ((e = cudaMemsetAsync(flags, 0, (size_t(ns) + 1) * 4, s)) != cudaSuccess) return e;
-        if (nflags && (e = cudaMemsetAsync(redo_flag, 0, nflags * 4, s)) != cudaSuccess) return e;
+        if (nflags && ((e = cudaMemsetAsync(call.redo_flag, 0, nflags * 4, s)) != cudaSuccess ||
+                       (e = cudaMemsetAsync(call.redo_queries_n, 0, 4, s)) != cudaSuccess))
+            return e;
         k_filter_mean<<<ns, 1024, 0, s>>>(call.X, d, ds, call.norms, mean);
         count_launch();
         k_filter_pack<<<unsigned((rows + 7) / 8), 256, 0, s>>>(
@@ -1119,7 +1128,8 @@ FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
             const int grid = int(std::min<uint32_t>(f.njobs, uint32_t(sms)));
             const uint32_t nb = r.b1 - r.b0;
             if ((e = launch_tiles<1>(nks, tmQ, tmC, f, grid, s)) != cudaSuccess) return e;
-            if ((e = launch_bound(max_chunks, ds, f.blocks, nb, minima, qn, abs_m, ath, s)) !=
+            if ((e = launch_bound(max_chunks, ds, f.blocks, nb, minima, qn, abs_m, flags, ath,
+                                  s)) !=
                 cudaSuccess)
                 return e;
             if ((e = launch_tiles<2>(nks, tmQ, tmC, f, grid, s)) != cudaSuccess) return e;

@@ -48,17 +48,19 @@ struct FilterCall {
     uint32_t* out_idx;
     float* out_dist;
     // queries the filter leaves to the full search, for every group:
-    //   FILTER_BATCHED: (group id, first query) blocks of redo_block queries,
-    //   and the single queries while there are few
-    //   else: query rows (redo_a)
-    std::vector<uint32_t> ids;  // FILTER_BATCHED: the caller's id of each group
+    //   FILTER_BATCHED: a flag per block of redo_block queries, and the single
+    //   queries while there are few
+    //   else: query rows
+    std::vector<uint32_t> ids;       // FILTER_BATCHED: the caller's id of each group
+    std::vector<uint64_t> redo_off;  //   and the first flag of its blocks
     uint32_t redo_block;
-    uint32_t* redo_a;    // device lists and their count (the caller's initial value is kept)
-    uint32_t* redo_b;
-    uint32_t* redo_count;
-    uint2* redo_queries;       // FILTER_BATCHED: (group id, query), the first redo_short of
-    uint32_t* redo_queries_n;  // redo_queries_n (zero before the call)
+    uint32_t* redo_flag;       // FILTER_BATCHED, device: redo_flags of them
+    uint64_t redo_flags;
+    uint2* redo_queries;       // FILTER_BATCHED, device: (group id, query), the first
+    uint32_t* redo_queries_n;  // redo_short of redo_queries_n
     uint32_t redo_short;
+    uint32_t* redo_rows;       // else, device: query rows and their number (zero before)
+    uint32_t* redo_rows_n;
 };
 
 // Plans the call and uploads the plan (workspace from the context); `run`
