@@ -767,13 +767,14 @@ int check_neighbors(pq_ctx* c, uint64_t n, uint64_t d, uint64_t nn, int32_t metr
 bool prepare_exact_filter(pq_ctx* c, const float* X, uint64_t n, uint64_t d, uint64_t kws,
                           int32_t metric, const float* norms, uint32_t* indices, float* dists,
                           pq::ExactFilter* out) {
-    if (kws < 2 || !pq::filter_takes(n, d, kws)) return false;
+    const int mode = metric == PQ_METRIC_COSINE ? pq::FILTER_COSINE : pq::FILTER_EUCLIDEAN;
+    if (kws < 2 || !pq::filter_takes(n, d, kws) || !pq::filter_pays(mode, n, d, kws)) return false;
     try {
         pq::FilterCall f{};
         f.X = X;
         f.rows = n;
         f.d = int(d);
-        f.mode = metric == PQ_METRIC_COSINE ? pq::FILTER_COSINE : pq::FILTER_EUCLIDEAN;
+        f.mode = mode;
         f.norms = metric == PQ_METRIC_COSINE ? norms : nullptr;
         pq::FilterSample s{};
         s.n = uint32_t(n);
@@ -1163,11 +1164,20 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
         // samples the tensor-core filter takes; the full search gets the rest,
         // and the query blocks the filter leaves (usually none)
         std::vector<uint8_t> taken(n_samples, 0);
-        uint64_t n_taken = 0;
+        uint64_t n_taken = 0, taken_points = 0, cost = 0, k_most = 0;
         for (uint32_t s = 0; s < n_samples; ++s) {
-            taken[s] = offsets[n_samples] < (uint64_t(1) << 30) &&
-                       pq::filter_takes(offsets[s + 1] - offsets[s], d, ks[s]);
-            n_taken += taken[s];
+            const uint64_t ns = offsets[s + 1] - offsets[s];
+            taken[s] =
+                offsets[n_samples] < (uint64_t(1) << 30) && pq::filter_takes(ns, d, ks[s]);
+            if (!taken[s]) continue;
+            ++n_taken;
+            taken_points += ns;
+            k_most = std::max<uint64_t>(k_most, ks[s]);
+            cost = std::max(cost, pq::batched_group_cost(ns, d, ks[s]));
+        }
+        if (!pq::filter_pays_batched(taken_points, d, k_most, cost)) {
+            taken.assign(n_samples, 0);
+            n_taken = 0;
         }
         if (it != c->batch_shape.end() && !(flags & PQ_BATCH_AUTOTUNE)) {
             shape = it->second;

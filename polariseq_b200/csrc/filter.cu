@@ -934,6 +934,31 @@ bool filter_takes(uint64_t n, uint64_t d, uint64_t k) {
            n < (uint64_t(1) << 30);
 }
 
+// A small group's search is a chain: each query is one warp that walks all
+// points, 1.3 ns per point and dimension (and 12 dimensions' worth besides), 28 us
+// in launches; the heap takes 3 us per neighbour.  The filter is ten launches, 80
+// us whatever the group, and under the cosine metric, whose FP32 distances tie
+// often, 3 us per neighbour for the queries that come back.  Whole calls, full
+// search and filter: 512 x 20, k = 6, 59 and 78 us; 700 x 50, k = 2, 76 and 82;
+// 1,000 x 20, k = 6, 84 and 82, cosine 92 and 108; 1,400 x 20, k = 6, 107 and 85,
+// cosine 118 and 113.  With less than 28 points per neighbour a small group's bound
+// is loose (8 columns per chunk at least) and its lists overflow: 512 x 20, k = 31,
+// 129 and 145 us; 1,000 x 20, 170 and 84.
+bool filter_pays(int mode, uint64_t n, uint64_t d, uint64_t k) {
+    const uint64_t walk = n * (d + 12);
+    if (mode == FILTER_COSINE) return walk + 330 * k >= 42000;
+    return walk + 2300 * k >= 46000 && (n >= 896 || n >= 28 * (k + 1));
+}
+// The same for a batch, whose full search spreads a group over the chip: 90 us for
+// the filter against 50 ns per point (90 ns above 32 dimensions) and 1.6 us per
+// neighbour of the largest group beside 40 us, until the batch fills the chip.
+// Whole calls without a graph: 4 x 512 x 20, k = 5, 75 and 96 us; 4 x 800 x 20, k =
+// 15, 109 and 100; 30 x 512 x 20, k = 5, 123 and 137, k = 15, 171 and 140; 30 x 800,
+// k = 5, 191 and 160.
+bool filter_pays_batched(uint64_t points, uint64_t d, uint64_t k, uint64_t group_cost) {
+    return group_cost >= 6200 || points + 500 * k >= (d <= 32 ? 20000 : 15000);
+}
+
 FilterPlan filter_prepare(pq_ctx* c, FilterCall call) {
     using pqh::ck;
     cudaStream_t st = c->stream;

@@ -37,6 +37,16 @@ enum { FILTER_BATCHED = 0, FILTER_EUCLIDEAN = 1, FILTER_COSINE = 2 };
 // k-th distance closely (16 points per neighbour), in at most 62 dimensions
 // (two columns of a 64-column operand block carry |x|^2 / 2).
 bool filter_takes(uint64_t n, uint64_t d, uint64_t k);
+// Whether it is faster than the full search for a group that it takes
+// (FILTER_EUCLIDEAN, FILTER_COSINE; k counts the point itself), or for a batch:
+// all its points, the largest k, and the cost of the group with the longest full
+// search.
+bool filter_pays(int mode, uint64_t n, uint64_t d, uint64_t k);
+bool filter_pays_batched(uint64_t points, uint64_t d, uint64_t k, uint64_t group_cost);
+// That search's time, in units of 10 ns.
+inline uint64_t batched_group_cost(uint64_t n, uint64_t d, uint64_t k) {
+    return n * (d <= 32 ? 5 : 9) + 160 * k;
+}
 
 struct FilterCall {
     const float* X;      // row-major rows, d floats each, any alignment

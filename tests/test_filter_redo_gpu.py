@@ -58,3 +58,28 @@ def test_exact_search_in_segments(n):
     ref = pq.neighbors_dense(wide(x), 9, "euclidean")
     np.testing.assert_array_equal(g["indices"], ref["indices"])
     assert g["data"].tobytes() == ref["data"].tobytes()
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+@pytest.mark.parametrize("n,d,k", [
+    (986, 20, 6), (1008, 20, 6), (1006, 20, 7),    # both sides of the rule at k = 6
+    (672, 50, 2), (688, 50, 2), (693, 50, 3),      # and at k = 2
+    (587, 30, 20), (588, 30, 20), (895, 12, 31), (896, 12, 31)])
+def test_exact_search_on_both_sides_of_the_rule(metric, n, d, k):
+    x = synth.mixture_dirichlet(n, d, 6, seed=n)
+    g = pq.neighbors_dense(x, k, metric)
+    ref = oracle.neighbors_exact(x, k, metric)
+    np.testing.assert_array_equal(g["indices"], ref["indices"])
+    assert g["data"].tobytes() == ref["data"].tobytes()
+
+
+@pytest.mark.parametrize("d", [32, 33])
+@pytest.mark.parametrize("count,n,k", [(1, 512, 22), (1, 512, 23), (1, 1079, 5), (1, 1080, 5),
+                                       (34, 512, 5), (24, 513, 5), (36, 514, 3), (30, 512, 15)])
+def test_batches_on_both_sides_of_the_rule(d, count, n, k):
+    xs = [synth.mixture_dirichlet(n, d, 5, seed=i) for i in range(count)]
+    got = pq.knn_batched(xs, [k] * count)
+    ref = pq.knn_batched([wide(x) for x in xs], [k] * count)
+    for (gi, gd), (ri, rd) in zip(got, ref):
+        np.testing.assert_array_equal(gi, ri)
+        assert gd.tobytes() == rd.tobytes()
