@@ -35,6 +35,7 @@
 
 #include "batched.cuh"
 #include "common.cuh"
+#include "seq_plan.cuh"
 
 namespace pq {
 namespace {
@@ -417,7 +418,7 @@ template <int DP, int QW, int NW, int KPL>
 cudaError_t launch_kpl(const BatchArgs& a, int sms, cudaStream_t st) {
     const size_t sm = smem_bytes<DP, QW, NW, KPL>(a.kp);
     cudaError_t e = cudaFuncSetAttribute(k_batched_knn<DP, QW, NW, KPL>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYNAMIC);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_knn<DP, QW, NW, KPL>,

@@ -452,10 +452,8 @@ void launch_sides(const ForestArgs& a, const PNode* nodes, const uint32_t* chunk
     const int rs = staged_stride(a.dp);
     size_t sm = size_t(a.dp) * 4, full = sm + size_t(FT) * rs * 4;
     const bool staged = full <= 100 * 1024;  // two CTAs per SM
-    if (staged) {
-        sm = full;
-        cudaFuncSetAttribute(k_sides, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
-    }
+    if (staged) sm = full;
+    cudaFuncSetAttribute(k_sides, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYNAMIC);
     k_sides<<<nchunks, FT, sm, st>>>(a, nodes, chunk_node, normals, chunkL, staged ? rs : 0);
     count_launch();
 }
@@ -501,13 +499,13 @@ void launch_leaf_pairs(const float* X, int d, int dp, const uint32_t* ids_t,
     if (d == 50) {
         if (sm > 40 * 1024)
             cudaFuncSetAttribute(k_leaf_pairs<50>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(sm));
+                                 SMEM_DYNAMIC);
         k_leaf_pairs<50><<<grid, LCAP, sm, st>>>(X, d, dp, ids_t, leaf_start, nleaves, n, k,
                                                  hidx, hdist, hflag, lmax, lpb); count_launch();
     } else {
         if (sm > 40 * 1024)
             cudaFuncSetAttribute(k_leaf_pairs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(sm));
+                                 SMEM_DYNAMIC);
         k_leaf_pairs<0><<<grid, LCAP, sm, st>>>(X, d, dp, ids_t, leaf_start, nleaves, n, k,
                                                 hidx, hdist, hflag, lmax, lpb); count_launch();
     }

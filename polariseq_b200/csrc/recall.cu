@@ -22,6 +22,7 @@
 
 #include "ctx.cuh"
 #include "kernels.cuh"
+#include "seq_plan.cuh"
 
 namespace pq {
 namespace {
@@ -248,15 +249,15 @@ double sampled_recall(pq_ctx* c, const float* X, int d, int dp, uint32_t n, int 
     if (reg) {
         const size_t sm2 = size_t(CH) * dp * sizeof(float);
         cudaFuncSetAttribute(k_sample_scan_reg<50>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(sm2));
+                             SMEM_DYNAMIC);
         k_sample_scan_reg<50><<<grid, QB, sm2, st>>>(X, dp, n, dq, Q, S, keys);
     } else if (d == 50) {
         cudaFuncSetAttribute(k_sample_scan<50>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(smem));
+                             SMEM_DYNAMIC);
         k_sample_scan<50><<<grid, SCAN_T, smem, st>>>(X, d, dp, n, dq, Q, S, keys);
     } else {
         cudaFuncSetAttribute(k_sample_scan<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(smem));
+                             SMEM_DYNAMIC);
         k_sample_scan<0><<<grid, SCAN_T, smem, st>>>(X, d, dp, n, dq, Q, S, keys);
     }
     count_launch();

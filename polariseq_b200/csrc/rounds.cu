@@ -11,6 +11,7 @@
 // replayed by one thread per destination row.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "seq_plan.cuh"
 
 namespace pq {
 namespace {
@@ -688,7 +689,8 @@ void launch_cand_apply(const uint32_t* keys, const uint64_t* vals, const uint32_
     }
     size_t sm = size_t(CREC) * 8 + size_t(m) * CT * 16;
     if (sm > 40 * 1024)
-        cudaFuncSetAttribute(k_cand_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+        cudaFuncSetAttribute(k_cand_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SMEM_DYNAMIC);
     k_cand_apply<<<(n + CT - 1) / CT, CT, sm, st>>>(keys, vals, seg_off, dcnt, n, m, new_idx,
                                                     new_prio, old_idx, old_prio); count_launch();
 }
@@ -705,7 +707,7 @@ static size_t join_smem_bytes(int m, int dp, int words) {
 template <class K>
 static void set_smem(K kern, size_t sm) {
     if (sm > 40 * 1024)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DYNAMIC);
 }
 
 void launch_join_count(const float* X, int d, int dp, uint32_t n, int k, int m,

@@ -17,6 +17,11 @@ namespace pq {
 
 // Shared memory a CTA may have (227 KB), static arrays included.
 constexpr size_t SMEM_PER_CTA = 232448;
+// A kernel's limit on dynamic shared memory belongs to the device, not to a
+// context: every launch sets the same limit, whatever it needs itself, so that
+// contexts on several threads do not lower each other's between setting and
+// launching.  (For kernels with less than 2 KB of static arrays.)
+constexpr int SMEM_DYNAMIC = int(SMEM_PER_CTA) - 2048;
 
 // Floats between staged rows of dp floats (dp a multiple of 4).
 PQ_PLAN int staged_stride(int dp) { return (dp / 4) % 2 ? dp : dp + 4; }

@@ -806,7 +806,7 @@ void seqtree_launch(const ForestArgs& a, const SRoot* roots, uint32_t nr, size_t
     const size_t dyn = seq_dynamic(a.dp, trows);
     // (with the static arrays the total passes 48 KB well before dyn does)
     cudaFuncSetAttribute(k_seqtree<NT, CAP, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(dyn));
+                         int(SMEM_PER_CTA - SEQ_FIXED<NT, CAP>));
     k_seqtree<NT, CAP, D><<<nr, NT, dyn, st>>>(a, roots, trows);
     count_launch();
 }
