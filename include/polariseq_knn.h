@@ -209,7 +209,13 @@ int pq_neighbors_into(pq_ctx* ctx, const float* data, uint64_t n_obs, uint64_t n
 
 /* The same with DEVICE buffers (data n_obs x n_dim row-major f32, any
  * alignment); `stream` (a cudaStream_t, may be null) is ordered before and
- * after the search.  The context's workspace holds the cosine row norms. */
+ * after the search.  The context's workspace holds the cosine row norms and,
+ * where the tensor-core filter answers (n_dim <= 62, at least 16 points per
+ * neighbour, not the smallest calls), its operands (128 or 256 bytes per row
+ * and operand, and two copies of the rows) and at most 2.6 GB of chunk maxima,
+ * lists and distances.  That part is optional: without room for it the full
+ * search answers, and any call of the context that needs the memory takes it
+ * back. */
 int pq_neighbors_into_device(pq_ctx* ctx, const float* d_data, uint64_t n_obs, uint64_t n_dim,
                              uint64_t n_neighbors, int32_t metric, uint32_t* d_indptr,
                              uint32_t* d_indices, float* d_dists, uint64_t* nnz_out,

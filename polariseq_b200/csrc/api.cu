@@ -770,6 +770,7 @@ bool prepare_exact_filter(pq_ctx* c, const float* X, uint64_t n, uint64_t d, uin
     const int mode = metric == PQ_METRIC_COSINE ? pq::FILTER_COSINE : pq::FILTER_EUCLIDEAN;
     if (kws < 2 || !pq::filter_takes(n, d, kws) || !pq::filter_pays(mode, n, d, kws)) return false;
     try {
+        FilterSetup setup(c);
         pq::FilterCall f{};
         f.X = X;
         f.rows = n;
@@ -795,6 +796,7 @@ bool prepare_exact_filter(pq_ctx* c, const float* X, uint64_t n, uint64_t d, uin
             64, std::min<uint64_t>((n + 7) / 8, (uint64_t(1) << 30) / (ld * 4)) / 4 * 4));
         out->redo_dist = c->get<float>(
             "ex_redo_d", std::max<uint64_t>(out->redo_cap * ld, pq::exact_redo_floats(uint32_t(ld))));
+        setup.done = true;
         return true;
     } catch (const std::string&) {
         return false;
@@ -1223,6 +1225,7 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
         std::function<cudaError_t(cudaStream_t)> filter;
         if (n_taken > 0) {
             try {
+                FilterSetup setup(c);
                 // the full search's items: those of the samples it takes whole, then
                 // those of the filter's samples, searched where the filter says so
                 items_for(shape, is, iq);
@@ -1278,6 +1281,7 @@ int pq_knn_batched_into_device(pq_ctx* c, const float* d_data, uint64_t d, uint3
                 const uint32_t* flag = f.redo_flag;
                 filter = pq::filter_prepare(c, std::move(f)).run;
                 b.flag = flag;
+                setup.done = true;
             } catch (const std::string&) {  // no room for the filter's workspace
                 filter = nullptr;
             }

@@ -121,6 +121,26 @@ struct pq_ctx {
     pq_ctx* sub = nullptr;
     pq::HostStage* stage = nullptr;  // pinned staging of large host copies
 
+    // Buffers of the exact searches' filter (the full search needs none of them)
+    // are named ft_..., ex_redo... and bt_redo...; in_filter: its set-up is
+    // collecting them, and the call falls back when one cannot be had.
+    bool in_filter = false;
+    // Frees them (no call in progress may hold one); false when there are none.
+    bool release_filter() {
+        bool any = false;
+        for (auto& kv : bufs) {
+            const std::string& s = kv.first;
+            if (!kv.second.p || (s.compare(0, 3, "ft_") && s.compare(0, 7, "ex_redo") &&
+                                 s.compare(0, 7, "bt_redo")))
+                continue;
+            if (!any) cudaStreamSynchronize(stream);
+            cudaFree(kv.second.p);
+            kv.second = pqh::Buf{};
+            any = true;
+        }
+        return any;
+    }
+
     template <class T>
     T* get(const std::string& name, size_t count) {
         size_t need = count * sizeof(T);
@@ -134,8 +154,15 @@ struct pq_ctx {
                 b.bytes = 0;
             }
             size_t alloc = need + need / 8;  // headroom for slightly larger calls
-            if (cudaMalloc(&b.p, alloc) != cudaSuccess) {
+            cudaError_t e = cudaMalloc(&b.p, alloc);
+            // the exact searches' filter can do without: its workspace makes room
+            if (e != cudaSuccess && !in_filter && release_filter()) {
                 cudaGetLastError();
+                e = cudaMalloc(&b.p, alloc);
+            }
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                b.p = nullptr;
                 throw std::string("device allocation of ") + std::to_string(alloc) +
                     " bytes failed (" + name + ")";
             }
@@ -146,6 +173,17 @@ struct pq_ctx {
 };
 
 namespace pqh {
+
+// The filter's set-up: what it has got is given back when it does not succeed.
+struct FilterSetup {
+    pq_ctx* c;
+    bool done = false;
+    explicit FilterSetup(pq_ctx* c_) : c(c_) { c->in_filter = true; }
+    ~FilterSetup() {
+        c->in_filter = false;
+        if (!done) c->release_filter();
+    }
+};
 
 // Brackets one kernel group with CUDA events on the context's stream when
 // profiling is on; the records are summed into the stats at the end.
