@@ -232,9 +232,17 @@ class Context:
         return {"indptr": oip, "indices": oix[:m], "data": ow[:m]}
 
     # -- host copies ---------------------------------------------------------
+    @staticmethod
+    def _check_copy(tensor, array: np.ndarray, offset: int) -> None:
+        if not array.flags.c_contiguous or not tensor.is_contiguous():
+            raise ValueError("host copies need contiguous arrays and tensors")
+        if offset < 0 or offset + array.nbytes > tensor.numel() * tensor.element_size():
+            raise ValueError("host copy past the end of the tensor")
+
     def copy_to_device(self, dst, src: np.ndarray, offset: int = 0, stream=None) -> None:
         """A contiguous array's bytes into the CUDA tensor `dst`, `offset` bytes
         in, after what `stream` still does with it."""
+        self._check_copy(dst, src, offset)
         sp = None if stream is None else C.c_void_p(int(stream))
         with self._lock:
             rc = _lib.load().pq_copy_to_device(self._h, dst.data_ptr() + offset, src.ctypes.data,
@@ -243,6 +251,7 @@ class Context:
 
     def copy_to_host(self, dst: np.ndarray, src, stream=None) -> None:
         """The first bytes of the CUDA tensor `src` into a contiguous array."""
+        self._check_copy(src, dst, 0)
         sp = None if stream is None else C.c_void_p(int(stream))
         with self._lock:
             rc = _lib.load().pq_copy_to_host(self._h, dst.ctypes.data, src.data_ptr(), dst.nbytes,
