@@ -2,12 +2,13 @@
 //
 // A brute-force search evaluates n distances per query in FP32 and keeps k of
 // them.  Here almost none of those distances is evaluated: two passes of
-// tcgen05 tiles over all pairs give every distance to within a proven bound,
-// and only the points that can be among the k nearest get the search's own
-// FP32 distance, so the result is the brute-force result, bit for bit.
+// tcgen05 tiles over all pairs give every distance to within a bound (derived
+// below, with one assumption about the accumulator), and only the points that can
+// be among the k nearest get the search's own FP32 distance, so the result is the
+// brute-force result, bit for bit.
 //
 //   mean, pack   coordinates centred on the group's mean (cosine: normalised
-//                rows), split into two BF16 parts hi + lo (2^-18 relative);
+//                rows), split into two BF16 parts hi + lo;
 //                candidate rows carry |x|^2 / 2 in three BF16 parts beside
 //                them, query rows the constants -1, so that
 //                  a = q.x - |x|^2 / 2 = (|q|^2 - |q - x|^2) / 2
@@ -22,14 +23,19 @@
 //                operation order, sorted by (distance, index)
 //
 // Bounds.  With A = |q|^2 - 2a and D the true squared distance, |A - D| is at
-// most e s^2, s = |q| + sqrt(D) >= |x|: the split drops lo.lo and both
-// residuals (3 x 2^-18 |q||x|, twice: 2.3e-5), the two norms are FP32 sums
-// (2^-18 each: 0.8e-5), and the accumulator adds the cross products first, at
-// 2^-9 of the magnitude, then at most 4 K = 16 steps of hi.hi, each charged 17
-// terms truncated at 2^-23 of a magnitude of at most 1.5 s^2 (twice: 2.4e-5):
-// e < 5.6e-5.  The FP32 distance itself is within 2^-17 D (cosine: 2^-17
-// absolute).  The margin, 2^-13 s^2 and those, takes both errors on both sides
-// of the comparison, s from the bound itself with 8 % to spare.
+// most e s^2, s = |q| + sqrt(D) >= |x|.  A BF16 part is within 2^-8 of its value
+// and the second part within 2^-17 of the binade's bottom, so dropping lo.lo and
+// the two residuals leaves 2^-16 + 2 x 2^-17 of |q||x| in a: 2^-14 |q||x| in A.
+// The norms' FP32 sums and the centring take 0.2e-5.  The accumulator adds the
+// cross products first, at 2^-8 of the magnitude, then at most 4 K = 16 steps of
+// hi.hi.  How tcgen05 rounds in between is not documented; ASSUMED is a
+// truncation of each of a step's 17 terms at 2^-23 of a magnitude of at most 1.5
+// s^2, 2.4e-5 in A.  Measured against FP64 (1 to 62 dimensions, both metrics,
+// normal, clustered, one-sided, count and heavy-tailed values): the accumulator
+// at most 1.7e-6, the sum of all 5.9e-5, against e < 8.8e-5.  The FP32 distance
+// itself is within 2^-17 D (cosine: 2^-17 absolute).  The margin, 3 x 2^-14 s^2
+// and those, takes both errors on both sides of the comparison; s from the bound
+// itself is short by 1.4 % at most.
 // A group with non-finite or huge rows, a list that overflows, an aborted
 // tile pass, and (for the heap-ordered searches) equal distances among the
 // k + 1 nearest send their queries to the full search.
@@ -559,7 +565,7 @@ __global__ void __launch_bounds__(256) k_filter_bound(const FilterSample* __rest
         const float n2 = qn[S.base + q];
         const float T = fmaxf(n2 - 2.0f * ta, 0.0f);
         const float s = sqrtf(n2) + sqrtf(T);
-        const float margin = 0x1p-13f * s * s + 0x1p-15f * T + abs_m;
+        const float margin = FILTER_MARGIN * s * s + 0x1p-15f * T + abs_m;
         // (a bound that is no number: everything is admitted and the list overflows)
         const float v = ta - 0.5f * margin;
         ath[b.slot + row] = v == v ? v : __int_as_float(0xff800000);

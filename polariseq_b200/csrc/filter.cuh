@@ -1,5 +1,5 @@
 // Tensor-core filter of the exact searches (filter.cu): which points can be
-// among a query's nearest, decided by rigorous bounds on split-BF16 distance
+// among a query's nearest, decided by bounds on split-BF16 distance
 // tiles; the survivors get the search's own FP32 distances.
 #pragma once
 

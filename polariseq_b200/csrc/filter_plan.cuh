@@ -49,6 +49,12 @@ PQ_PLAN uint32_t filter_chunk_log(uint32_t n, uint32_t tiles, uint32_t ksel) {
     return lc;
 }
 
+// The admission margin, in units of s^2 = (|q| + sqrt(D))^2, and the error of an
+// approximate squared distance in them that it has to cover twice (filter.cu).
+constexpr float FILTER_MARGIN = 3.0f / 16384.0f;
+constexpr double FILTER_ERROR_SPLIT = 1.0 / 16384.0;  // the BF16 parts, in |q| |x| <= s^2
+constexpr double FILTER_ERROR_SUMS = 2.6e-5;          // the FP32 norms and the accumulator
+
 // Tiles per job when a query block's candidates are cut into at most `want`
 // slices: whole chunks, and at least two tiles.
 PQ_PLAN uint32_t filter_slice_tiles(uint32_t tiles, uint32_t logc, uint32_t want) {
