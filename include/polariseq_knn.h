@@ -267,18 +267,23 @@ int pq_copy_to_host(pq_ctx* ctx, void* dst, const void* d_src, uint64_t bytes, v
 enum { PQ_BATCH_AUTOTUNE = 1, PQ_BATCH_GRAPH = 2 };
 
 /* Batched exact kNN: every point's k_s nearest other points within its own
- * sample, for n_samples samples of uneven size in ONE persistent,
- * work-queued launch — the per-sample searches of doublet scoring
+ * sample, for n_samples samples of uneven size in one call — the per-sample
+ * searches of doublet scoring
  * (crates/polariseq-core/src/doublets.rs:544-650 knn_exact: exact, itself
  * excluded, ties by index, ascending).  d_data holds all samples' rows back
  * to back (row-major f32, n_dim <= 64); offsets (HOST, n_samples + 1, rows)
  * delimit the samples; ks (HOST) gives each sample's k (1 <= k < its size,
  * k <= 512).  Sample s's rows write k_s entries each, back to back from
  * sum_{t<s} n_t * k_t: indices local to the sample, Euclidean distances.
- * PQ_BATCH_AUTOTUNE re-times the tile shapes (otherwise the context's choice
- * for this n_dim and k range is reused, timing them on first use);
- * PQ_BATCH_GRAPH captures the launch in a CUDA graph and replays it.
- * *shape_out (may be null) receives the tile shape used. */
+ * Where it applies (n_dim <= 62, samples with at least 16 points per neighbour,
+ * not the smallest calls) the tensor-core filter answers, all samples together
+ * in a few launches; ONE persistent, work-queued launch of the full search takes
+ * the other samples and the queries that the filter leaves.
+ * PQ_BATCH_AUTOTUNE re-times the full search's tile shapes (otherwise the
+ * context's choice for this n_dim and k range is reused; calls that need the
+ * full search for whole samples time the shapes on first use);
+ * PQ_BATCH_GRAPH captures the launches in a CUDA graph and replays it.
+ * *shape_out (may be null) receives the tile shape of the full search. */
 int pq_knn_batched_into_device(pq_ctx* ctx, const float* d_data, uint64_t n_dim,
                                uint32_t n_samples, const uint64_t* offsets, const uint32_t* ks,
                                uint32_t* d_indices, float* d_dists, int32_t flags,
@@ -294,7 +299,7 @@ int pq_knn_batched_into_device(pq_ctx* ctx, const float* d_data, uint64_t n_dim,
  * indices local to the sample).  Each sample's points are its cells
  * (w u - mv) and doublets (1e6 / (total_x + total_y) (u_x + u_y) - mv) in f32
  * from f64 arithmetic in the reference's order; the exact kNN of every point
- * within its sample runs in one persistent launch (pq_knn_batched_into_device)
+ * within its sample, all samples in one call (pq_knn_batched_into_device),
  * with k_adj = round_half_even(k (1 + n_sim / n)) neighbours; every point's
  * score is the reference's Bayesian score from its simulated neighbours
  * (q = (n_d + 1) / (k_adj + 2), rho the expected doublet rate), f64 into

@@ -382,7 +382,7 @@ def fuzzy_connectivities(indptr, indices, data, n_obs, *, device: int = 0) -> di
 
 
 def knn_batched(samples, ks, *, device: int = 0, autotune: bool = False, graph: bool = True):
-    """Exact kNN within each sample, all samples in one persistent launch
+    """Exact kNN within each sample, all samples in one call
     (the per-sample search of doublet scoring, doublets.rs:544-650).
 
     ``samples``: list of float32 [n_s, d] arrays (d <= 64); ``ks``: the k of

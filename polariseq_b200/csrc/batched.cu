@@ -21,7 +21,8 @@
 // the root when a key is smaller, lanes visited in index order) and sorted
 // by a warp bitonic network at the end.  Either way the result is the exact k
 // smallest keys.  The tile shape (QW, NW) is chosen by an autotuner that
-// times each shape on the largest work items of the call.
+// times each shape on the largest work items of the call, or by a rule on k and
+// the number of points where the filter takes every sample.
 //
 // This full search takes the samples the tensor-core filter (filter.cu) does
 // not: d > 62 or fewer than 16 points per neighbour; and the query blocks that

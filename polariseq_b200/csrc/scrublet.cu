@@ -6,7 +6,7 @@
 //      order (no fused multiply-add): cell i -> w_i u_i - mv, doublet (x, y)
 //      -> s (u_x + u_y) - mv with s = 1e6 / (totals_x + totals_y);
 //   2. the exact kNN of every point within its sample, all samples in one
-//      persistent launch (pq_knn_batched_into_device; (distance, index)
+//      call (pq_knn_batched_into_device; (distance, index)
 //      order, as knn_exact), k_adj = round_half_even(k (1 + r)), r = n_sim/n;
 //   3. k_scrublet_score: the Bayesian score from the count of simulated
 //      neighbours, q = (n_d + 1) / (k_adj + 2),
